@@ -89,22 +89,29 @@ std::mutex g_tune_mu;
 std::map<std::tuple<int, int, int>, int> g_tune_cache;
 }  // namespace
 
+int forced_tile_rows() {
+  const char* e = std::getenv("AUSM_TILE_ROWS");
+  const int r = e ? std::atoi(e) : 0;
+  return r == 8 || r == 16 || r == 32 ? r : 0;
+}
+
 int tuned_tile_rows(ausm_solver* h, bool force, int* rows) {
   *rows = 16;
   if (!h->tma[1].ok) return AUSM_OK;  // per-thread kernels: 16 rows
-  if (const char* e = std::getenv("AUSM_TILE_ROWS")) {
-    const int r = std::atoi(e);
-    if ((r == 8 || r == 16 || r == 32) && h->tma[tile_index(r)].ok) {
+  if (const int r = forced_tile_rows())
+    if (h->tma[tile_index(r)].ok) {
       *rows = r;
       return AUSM_OK;
     }
-  }
   if (const char* e = std::getenv("AUSM_AUTOTUNE"))
     if (e[0] == '0') return AUSM_OK;
   if (!force && h->tile_rows) {
     *rows = h->tile_rows;
     return AUSM_OK;
   }
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(h->st, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone)
+    return AUSM_OK;  // a grid whose steps have all been resident so far: not tuned yet
   const auto key = std::make_tuple(h->M, h->N, h->p.scheme);
   if (!force) {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -388,6 +395,7 @@ int ausm_destroy(ausm_solver* h) {
   if (!h) return AUSM_OK;
   if (h->batch) ausm_batch_remove(h->batch, h);
   cudaSetDevice(h->dev);
+  if (h->counted) resident_user(h->dev, -1);
   if (h->st) cudaStreamSynchronize(h->st);
   void* dptrs[] = {h->V, h->V2, h->Vd, h->Mi, h->Mj, h->Q[0], h->Q[1], h->Q[2], h->S[0], h->S[1], h->S[2], h->fx, h->fy, h->res,
                    h->flen, h->area, h->staging, h->cp, h->wave, h->dt, h->dacc, h->parts, h->move, h->err_flag};
@@ -458,6 +466,8 @@ int ausm_create(int M, int N, ausm_solver** out) {
     // a solve whose maps cannot be encoded steps with the per-thread staging kernel
     for (int k = 0; k < 3; k++) encode_tma_maps(qs, h->Mi, h->Mj, M, N, kTileHeights[k], &h->tma[k]);
   }
+  resident_user(h->dev, 1);
+  h->counted = true;
   ausm_default_params(&h->p);
   h->speed_now = inflow_target(h->p);
   make_consts(h);
@@ -789,6 +799,42 @@ int ausm_get_state_f64(ausm_solver* h, double* q) {
 }  // extern "C"
 
 namespace {
+// After dt and the max wave speed have been queued to h_dt and h_wave: waits and checks them.
+int read_dt(ausm_solver* h, float* dt_out) {
+  int rc = sync_and_check(h);
+  if (rc) return rc;
+  *dt_out = h->h_dt[0];
+  if (!std::isfinite(h->h_dt[1]) || !std::isfinite(h->h_dt[0]))
+    return fail(h, AUSM_ERR_DIVERGED, "max wave speed is not finite: the solution diverged");
+  return AUSM_OK;
+}
+
+// Tile height of the resident kernel for h's next steps, 0: the stage kernels.  A stream
+// capture stays on those: a captured launch would hold an exchange buffer that others use.
+int resident_height(ausm_solver* h, int* rows) {
+  *rows = 0;
+  if (forced_tile_rows()) return AUSM_OK;
+  const int r = resident_rows(resident_tiles(h->M, h->N, 4), resident_tiles(h->M, h->N, 8));
+  if (!r) return AUSM_OK;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  CU(h, cudaStreamIsCapturing(h->st, &cap));
+  if (cap == cudaStreamCaptureStatusNone) *rows = r;
+  return AUSM_OK;
+}
+
+// n fused steps by the resident kernel.
+int resident_steps(ausm_solver* h, int n, int rows) {
+  for (int done = 0; done < n;) {
+    const int k = std::min(n - done, kResidentSteps);
+    const int to = (h->cur + k) % 3;
+    CU(h, launch_resident(h->p.scheme, h->Q[h->cur], h->Q[to], h->Mi, h->Mj, h->dt, h->wave, rows, k, done == 0,
+                          done + k == n, h->h_dt, (int*)h->h_wave + 2, h->err_flag, h->c, h->M, h->N, h->st));
+    h->cur = to;
+    done += k;
+  }
+  return AUSM_OK;
+}
+
 // ausm_step; read_err: queue the read of the timeout flag (ausm_time_steps queues one
 // after all its repetitions instead, so that its timed steps stay back to back).
 int step_impl(ausm_solver* h, int n, float* dt_out, bool read_err) {
@@ -812,6 +858,14 @@ int step_impl(ausm_solver* h, int n, float* dt_out, bool read_err) {
         return fail(h, AUSM_ERR_DIVERGED, "max wave speed is not finite: the solution diverged");
     }
     return AUSM_OK;
+  }
+  int res_rows = 0;
+  if (h->engine == AUSM_ENGINE_FUSED && n > 0 && (rc = resident_height(h, &res_rows))) return rc;
+  if (res_rows) {
+    if ((rc = resident_steps(h, n, res_rows))) return rc;
+    ramp_after_steps(h, n);
+    h->err_read_queued = true;
+    return dt_out ? read_dt(h, dt_out) : AUSM_OK;
   }
   if (n == 0 || h->engine != AUSM_ENGINE_FUSED) launch_dt(h->wave, h->dt, h->c.maxdt, h->c.cfl, s);
   if (n > 0) {
@@ -865,13 +919,8 @@ int step_impl(ausm_solver* h, int n, float* dt_out, bool read_err) {
   if (h->engine == AUSM_ENGINE_FUSED && n > 0 && (read_err || dt_out) && (rc = queue_err_read(h))) return rc;
   if (dt_out) {
     CU(h, cudaMemcpyAsync(h->h_dt, h->dt, sizeof(float), cudaMemcpyDeviceToHost, s));
-    CU(h, cudaMemcpyAsync(h->h_wave, h->wave, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    if ((rc = sync_and_check(h))) return rc;
-    *dt_out = h->h_dt[0];
-    float w;
-    std::memcpy(&w, h->h_wave, 4);
-    if (!std::isfinite(w) || !std::isfinite(h->h_dt[0]))
-      return fail(h, AUSM_ERR_DIVERGED, "max wave speed is not finite: the solution diverged");
+    CU(h, cudaMemcpyAsync(h->h_dt + 1, h->wave, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    return read_dt(h, dt_out);
   }
   return AUSM_OK;
 }
@@ -1008,6 +1057,7 @@ int ausm_debug_set_wait_polls(unsigned polls) {
   cudaError_t e = cudaDeviceSynchronize();
   if (e == cudaSuccess) e = set_wait_polls_fused(polls);
   if (e == cudaSuccess) e = set_wait_polls_batch(polls);
+  if (e == cudaSuccess) e = set_wait_polls_resident(polls);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e != cudaSuccess) return fail(nullptr, AUSM_ERR_CUDA, std::string("wait polls: ") + cudaGetErrorString(e));
   return AUSM_OK;

@@ -133,6 +133,7 @@ struct BatchSolve {
   Consts c;
   int M, N, scheme, tiles_x, tile0, cur;  // scheme: the work-list group key (scheme, + 4 with MUSCL on)
   int chunk0;  // first residual-norm chunk (512 cells) of the solve
+  int rtile0;  // first tile of the solve in a resident launch
 };
 // Tensor maps per batch member, in this order: halo[0..2], plain[0..2], mi, mj,
 // wrap[0..2] (TmaMaps of the batch's tile height).
@@ -165,6 +166,31 @@ void launch_batch_gather(const BatchSolve* d, int nsolves, float* out, cudaStrea
 // descriptors).  Summation order depends only on the solve's own grid.
 void launch_batch_residual_norm(const BatchSolve* d, int nsolves, int total_chunks, double* part, double* l2,
                                 cudaStream_t s);
+
+// ---- resident engine (kernels_resident.cu): all steps of a call in one launch ----
+// Tile height (4 or 8) of a resident launch over `tiles4` tiles of 4 rows or `tiles8` of 8
+// (sums of resident_tiles over its solves); 0 when they do not all fit on the chip at once.
+int resident_rows(int tiles4, int tiles8);
+int resident_tiles(int M, int N, int rows);
+// nsteps steps from Qs to Qo (which may be the same buffer).  first: dt from wave[0], else
+// *dt; last: the new state's max wave speed to wave[0].  wave: 3 words, see Job in
+// kernels_resident.cu.  out (dt, wave speed) and out_err (*err) are written at the end, in
+// pinned host memory or null.
+cudaError_t launch_resident(int scheme, const float4* Qs, float4* Qo, const float4* Mi, const float4* Mj, float* dt,
+                            uint32_t* wave, int rows, int nsteps, bool first, bool last, float* out, int* out_err,
+                            int* err, const Consts& c, int M, int N, cudaStream_t s);
+// The same for a batch: items[k] = (descriptor, tile of that solve); every solve goes from
+// Q[cur] to Q[(cur + nsteps) % 3].
+cudaError_t launch_resident_batch(const BatchSolve* solves, const int2* items, int tiles, int rows, int nsolves,
+                                  int nsteps, bool first, bool last, int* err, cudaStream_t s);
+cudaError_t set_wait_polls_resident(unsigned polls);
+// Counts the solvers and batches of a device (+1, -1); with the last one its exchange
+// buffers are freed.
+void resident_user(int dev, int change);
+// Steps of one resident launch at most (10 ms on the largest grids it takes), so that it
+// does not keep the chip from other streams for long; a multiple of 3, so that the buffers
+// rotate as they do step by step.
+constexpr int kResidentSteps = 2049;
 
 // ---- full-FP64 engine (kernels_f64.cu, built with -fmad=false) ----
 // The reference-shaped engine in double on its own buffers; vertices are the solver's

@@ -44,8 +44,8 @@ struct ausm_batch {
     int scheme, s_lo, s_hi, t_lo, t_hi;  // group key (group_key), descriptors [s_lo, s_hi), items [t_lo, t_hi)
   };
   std::vector<Group> groups;
-  cudaStream_t aux[2] = {nullptr, nullptr};  // branches of the second and third group
-  cudaEvent_t fork = nullptr, join[2] = {nullptr, nullptr};
+  cudaStream_t aux[5] = {};  // branches of the second group and on (3 schemes x MUSCL on or off)
+  cudaEvent_t fork = nullptr, join[5] = {};
   bool uploaded = false;
   int total_tiles = 0;
   int total_chunks = 0;  // residual-norm chunks of all members
@@ -57,10 +57,15 @@ struct ausm_batch {
   CUtensorMap* d_maps = nullptr;  // kBatchMaps per descriptor when tma
   bool tma = false;               // every member has tensor maps: stages load tiles by TMA
   int rows = 16;                  // tile height of the work list
+  int res_rows = 0;               // tile height of resident launches, 0: the members do not fit
+  std::vector<int2> ritems;       // their work items (the device's d_ritems)
+  int2* d_ritems = nullptr;
+  int ritem_cap = 0;
   int tuned_rows = 0;             // height chosen by the last tuning run (0: none yet)
   double tuned_cells = 0.0;       // the batch's cell count at that run
   int* d_err = nullptr;           // set by a TMA tile whose bounded wait gave up
   int* h_err = nullptr;           // pinned copy of *d_err
+  bool counted = false;           // a user of the device's exchange buffers (resident_user)
   bool err_read_queued = false;   // a copy of *d_err to *h_err is queued on st
   int cap = 0;  // descriptor capacity of d_solves / d_maps / d_out / d_l2
   float* d_out = nullptr;
@@ -112,9 +117,10 @@ void drop_graphs(ausm_batch* b) {
 // kernels are then instantiated with MUSCL known on, without a per-face branch).
 int group_key(const ausm_solver* h) { return h->p.scheme + (h->p.muscl > 0 ? 4 : 0); }
 
-BatchSolve describe(const ausm_solver* h, int tile0, int chunk0, const CUtensorMap* maps) {
+BatchSolve describe(const ausm_solver* h, int tile0, int chunk0, int rtile0, const CUtensorMap* maps) {
   BatchSolve d{};
   d.chunk0 = chunk0;
+  d.rtile0 = rtile0;
   d.maps = maps;
   for (int k = 0; k < 3; k++) d.Q[k] = h->Q[k];
   d.Mi = h->Mi;
@@ -135,8 +141,14 @@ const CUtensorMap* maps_of(const ausm_batch* b, int k) {
   return b->tma ? b->d_maps + ausm::kBatchMaps * (size_t)k : nullptr;
 }
 
-// Grows the per-member and per-tile device arrays (dropping graphs that point at them).
+// Grows the per-member and per-tile device arrays (dropping graphs that point at them) and
+// the groups' branch streams.
 int ensure_capacity(ausm_batch* b) {
+  for (int g = 0; g + 1 < (int)b->groups.size(); g++)
+    if (!b->join[g]) {
+      BCU(b, cudaStreamCreateWithFlags(&b->aux[g], cudaStreamNonBlocking));
+      BCU(b, cudaEventCreateWithFlags(&b->join[g], cudaEventDisableTiming));
+    }
   const int n = (int)b->members.size();
   if (n > b->cap) {
     int cap = std::max(n, 2 * b->cap);
@@ -170,6 +182,16 @@ int ensure_capacity(ausm_batch* b) {
     b->item_cap = cap;
     b->uploaded = false;
   }
+  if ((int)b->ritems.size() > b->ritem_cap) {
+    int cap = std::max((int)b->ritems.size(), 2 * b->ritem_cap);
+    BCU(b, cudaStreamSynchronize(b->st));
+    cudaFree(b->d_ritems);
+    b->d_ritems = nullptr;
+    b->ritem_cap = 0;
+    BCU(b, cudaMalloc((void**)&b->d_ritems, cap * sizeof(int2)));
+    b->ritem_cap = cap;
+    b->uploaded = false;
+  }
   if (b->total_chunks > b->part_cap) {
     int cap = std::max(b->total_chunks, 2 * b->part_cap);
     BCU(b, cudaStreamSynchronize(b->st));
@@ -201,12 +223,23 @@ void relayout(ausm_batch* b) {
   for (ausm_solver* h : b->members) b->tma = b->tma && h->tma[0].ok && h->tma[1].ok && h->tma[2].ok;
   if (!b->tma) b->rows = 16;
   const int rows = b->rows;
+  int tiles4 = 0, tiles8 = 0;
+  for (ausm_solver* h : b->members) {
+    tiles4 = std::min(1 << 20, tiles4 + ausm::resident_tiles(h->M, h->N, 4));
+    tiles8 = std::min(1 << 20, tiles8 + ausm::resident_tiles(h->M, h->N, 8));
+  }
+  b->res_rows = b->members.empty() ? 0 : ausm::resident_rows(tiles4, tiles8);
+  b->ritems.clear();
   int chunks = 0;
   for (int k : b->order) {
     const ausm_solver* h = b->members[k];
     const int s = (int)b->mirror.size();
     if (b->groups.empty() || b->groups.back().scheme != group_key(h)) b->groups.push_back({group_key(h), s, s, t, t});
-    b->mirror.push_back(describe(h, t, chunks, maps_of(b, s)));
+    b->mirror.push_back(describe(h, t, chunks, (int)b->ritems.size(), maps_of(b, s)));
+    if (b->res_rows) {
+      const int nt = ausm::resident_tiles(h->M, h->N, b->res_rows);
+      for (int k = 0; k < nt; k++) b->ritems.push_back(make_int2(s, k));
+    }
     const int tx = (h->M + kTX - 1) / kTX, tiles = tx * ((h->N + rows - 1) / rows);
     for (int k = 0; k < tiles; k++) b->items.push_back({s, 0, (k % tx) | (k / tx) << 16, h->M});
     t += tiles;
@@ -226,9 +259,11 @@ int sync_descriptors(ausm_batch* b) {
       relayout(b);
       break;
     }
+  if (int rc = ensure_capacity(b)) return rc;  // fewer members may have more (resident) work items
   bool changed = !b->uploaded;
   for (size_t k = 0; k < b->members.size(); k++) {
-    BatchSolve d = describe(b->members[b->order[k]], b->mirror[k].tile0, b->mirror[k].chunk0, maps_of(b, (int)k));
+    BatchSolve d = describe(b->members[b->order[k]], b->mirror[k].tile0, b->mirror[k].chunk0, b->mirror[k].rtile0,
+                            maps_of(b, (int)k));
     if (std::memcmp(&d, &b->mirror[k], sizeof d) != 0) {
       b->mirror[k] = d;
       changed = true;
@@ -257,6 +292,9 @@ int sync_descriptors(ausm_batch* b) {
     BCU(b, cudaMemcpyAsync(b->d_items, b->items.data(), b->items.size() * sizeof(ausm::BatchItem),
                            cudaMemcpyHostToDevice, b->st));
     BCU(b, cudaMemsetAsync(b->d_steps, 0, sizeof(int), b->st));
+    if (!b->ritems.empty())
+      BCU(b, cudaMemcpyAsync(b->d_ritems, b->ritems.data(), b->ritems.size() * sizeof(int2), cudaMemcpyHostToDevice,
+                             b->st));
     b->uploaded = true;
   }
   return AUSM_OK;
@@ -374,6 +412,22 @@ int sync_and_check(ausm_batch* b) {
   return bfail(b, AUSM_ERR_TIMEOUT, "a tile load did not arrive within the bounded wait");
 }
 
+// n steps of every member by resident launches, then the rotation and the gather as in
+// enqueue_steps.
+int resident_steps(ausm_batch* b, int n) {
+  const int ns = (int)b->members.size();
+  for (int done = 0; done < n;) {
+    const int k = std::min(n - done, ausm::kResidentSteps);
+    BCU(b, ausm::launch_resident_batch(b->d_solves, b->d_ritems, (int)b->ritems.size(), b->res_rows, ns, k, done == 0,
+                                       done + k == n, b->d_err, b->st));
+    ausm::launch_batch_advance(b->d_solves, ns, k, b->d_steps, b->st);
+    done += k;
+  }
+  ausm::launch_batch_gather(b->d_solves, ns, b->d_out, b->st);
+  BCU(b, cudaGetLastError());
+  return AUSM_OK;
+}
+
 int run_steps(ausm_batch* b, int n) {
   if (!b->graphs) {
     enqueue_steps(b, n);
@@ -421,12 +475,6 @@ int ausm_batch_create(ausm_batch** out) {
   if (e != cudaSuccess) return bail(e, "cudaStreamCreateWithFlags");
   if ((e = cudaEventCreate(&b->e0)) != cudaSuccess || (e = cudaEventCreate(&b->e1)) != cudaSuccess)
     return bail(e, "cudaEventCreate");
-  for (int g = 0; g < 2; g++) {
-    e = cudaStreamCreateWithFlags(&b->aux[g], cudaStreamNonBlocking);
-    if (e != cudaSuccess) return bail(e, "cudaStreamCreateWithFlags");
-    e = cudaEventCreateWithFlags(&b->join[g], cudaEventDisableTiming);
-    if (e != cudaSuccess) return bail(e, "cudaEventCreate");
-  }
   e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
   if (e != cudaSuccess) return bail(e, "cudaEventCreate");
   if ((e = cudaMalloc((void**)&b->d_err, 2 * sizeof(int))) != cudaSuccess) return bail(e, "cudaMalloc");
@@ -434,6 +482,8 @@ int ausm_batch_create(ausm_batch** out) {
   *b->h_err = 0;
   if ((e = cudaMemsetAsync(b->d_err, 0, 2 * sizeof(int), b->st)) != cudaSuccess) return bail(e, "cudaMemsetAsync");
   b->d_steps = b->d_err + 1;
+  ausm::resident_user(b->dev, 1);
+  b->counted = true;
   *out = b;
   return AUSM_OK;
 }
@@ -446,6 +496,7 @@ int ausm_batch_destroy(ausm_batch* b) {
   drop_graphs(b);
   cudaFree(b->d_solves);
   cudaFree(b->d_items);
+  cudaFree(b->d_ritems);
   cudaFree(b->d_maps);
   cudaFree(b->d_err);
   cudaFree(b->d_out);
@@ -457,7 +508,7 @@ int ausm_batch_destroy(ausm_batch* b) {
   if (b->e0) cudaEventDestroy(b->e0);
   if (b->e1) cudaEventDestroy(b->e1);
   if (b->fork) cudaEventDestroy(b->fork);
-  for (int g = 0; g < 2; g++) {
+  for (int g = 0; g < 5; g++) {
     if (b->aux[g]) {
       cudaStreamSynchronize(b->aux[g]);
       cudaStreamDestroy(b->aux[g]);
@@ -465,6 +516,7 @@ int ausm_batch_destroy(ausm_batch* b) {
     if (b->join[g]) cudaEventDestroy(b->join[g]);
   }
   if (b->st) cudaStreamDestroy(b->st);
+  if (b->counted) ausm::resident_user(b->dev, -1);
   delete b;
   return AUSM_OK;
 }
@@ -527,11 +579,13 @@ int batch_step_impl(ausm_batch* b, int n, float* dt_wave, bool read_err) {
   if (ns == 0 || n == 0) return AUSM_OK;
   for (ausm_solver* h : b->members)
     BNEED(b, h->has_grid && h->has_state, AUSM_ERR_STATE, "a member lost its grid or state");
-  rc = tune_rows(b);
-  if (rc) return rc;
+  // members whose tiles all fit on the chip together step in one launch
+  const bool fixed = ausm::forced_tile_rows() != 0;
+  if ((fixed || !b->res_rows) && (rc = tune_rows(b))) return rc;
   rc = sync_descriptors(b);
   if (rc) return rc;
-  rc = run_steps(b, n);
+  const bool resident = !fixed && b->res_rows != 0;
+  rc = resident ? resident_steps(b, n) : run_steps(b, n);
   if (rc) return rc;
   for (size_t k = 0; k < b->members.size(); k++) {
     ausm_solver* h = b->members[b->order[k]];
@@ -539,7 +593,7 @@ int batch_step_impl(ausm_batch* b, int n, float* dt_wave, bool read_err) {
     b->mirror[k].cur = h->cur;  // the device advanced its copy
     ausm::ramp_after_steps(h, n);
   }
-  if (b->tma && (read_err || dt_wave) && (rc = queue_err_read(b))) return rc;
+  if ((b->tma || resident) && (read_err || dt_wave) && (rc = queue_err_read(b))) return rc;
   if (!dt_wave) return AUSM_OK;
   BCU(b, cudaMemcpyAsync(b->h_out, b->d_out, ns * 2 * sizeof(float), cudaMemcpyDeviceToHost, b->st));
   if ((rc = sync_and_check(b))) return rc;
@@ -592,7 +646,7 @@ int ausm_batch_time_steps(ausm_batch* b, int n, int reps, float* ms_out) {
     if (rc) return rc;
   }
   BCU(b, cudaEventRecord(b->e1, b->st));
-  if (b->tma && (rc = queue_err_read(b))) return rc;
+  if ((rc = queue_err_read(b))) return rc;
   BCU(b, cudaEventSynchronize(b->e1));
   BCU(b, cudaEventElapsedTime(ms_out, b->e0, b->e1));
   return sync_and_check(b);

@@ -33,7 +33,7 @@ struct ausm_solver {
   float* area = nullptr;
   float4* staging = nullptr;
   double* cp = nullptr;
-  uint32_t* wave = nullptr;
+  uint32_t* wave = nullptr;    // [0] max wave speed bits; [1..2] the resident kernel's (kernels_resident.cu)
   float* dt = nullptr;
   double* dacc = nullptr;
   double* parts = nullptr;  // 2 * kMaxParts per-block partial sums
@@ -41,6 +41,7 @@ struct ausm_solver {
   int* err_flag = nullptr;  // set by a kernel whose bounded wait gave up
   bool err_read_queued = false;  // a copy of *err_flag to h_wave[2] is queued on st (api.cu)
   ausm::TmaMaps tma[3];  // per tile height kTileHeights[k]
+  bool counted = false;   // a user of the device's exchange buffers (resident_user)
   int tile_rows = 0;      // tile height of the TMA stage kernel; 0 until tuned
   float* h_dt = nullptr;
   uint32_t* h_wave = nullptr;
@@ -57,6 +58,9 @@ void set_thread_error(const std::string& msg);
 // Tile height for h's fused steps: AUSM_TILE_ROWS, the process-wide tuning cache for
 // (M, N, scheme), or a tuning run (api.cu).  Enqueues work on h's stream; must not run
 // inside a stream capture.
+// The tile height AUSM_TILE_ROWS fixes for the stage kernels (8, 16 or 32), or 0.  A fixed
+// height also keeps small grids on the stage kernels.
+int forced_tile_rows();
 int tuned_tile_rows(ausm_solver* h, bool force, int* rows);
 inline int tile_index(int rows) { return rows == 8 ? 0 : (rows == 32 ? 2 : 1); }
 }  // namespace ausm
