@@ -397,7 +397,7 @@ int ausm_destroy(ausm_solver* h) {
   cudaSetDevice(h->dev);
   if (h->counted) resident_user(h->dev, -1);
   if (h->st) cudaStreamSynchronize(h->st);
-  void* dptrs[] = {h->V, h->V2, h->Vd, h->Mi, h->Mj, h->Q[0], h->Q[1], h->Q[2], h->S[0], h->S[1], h->S[2], h->fx, h->fy, h->res,
+  void* dptrs[] = {h->V, h->Vd, h->Mi, h->Mj, h->Q[0], h->Q[1], h->Q[2], h->S[0], h->S[1], h->S[2], h->fx, h->fy, h->res,
                    h->flen, h->area, h->staging, h->cp, h->wave, h->dt, h->dacc, h->parts, h->move, h->err_flag};
   for (void* d : dptrs)
     if (d) cudaFree(d);
@@ -638,51 +638,47 @@ int ausm_generate_grid(ausm_solver* h, int iters, int method, double tol, int* i
   if (rc) return rc;
   const int M = h->M, N = h->N;
   int done = 0;
+  // the boundary rows go up; the guess fills the others
   if (method == AUSM_GRID_JACOBI) {  // FP32, the reference's generator (shaders/grid.js:33-113)
-    std::vector<float> v((size_t)M * (N + 1) * 2, 0.0f);
-    for (int i = 0; i < M; i++) {
-      v[2 * i] = (float)h->body[2 * i];
-      v[2 * i + 1] = (float)h->body[2 * i + 1];
-      size_t o = ((size_t)N * M + i) * 2;
-      v[o] = (float)h->outer[2 * i];
-      v[o + 1] = (float)h->outer[2 * i + 1];
+    std::vector<float> v((size_t)M * 4);
+    for (int i = 0; i < 2 * M; i++) {
+      v[i] = (float)h->body[i];
+      v[2 * M + i] = (float)h->outer[i];
     }
-    CU(h, cudaMemcpyAsync(h->V, v.data(), v.size() * sizeof(float), cudaMemcpyHostToDevice, h->st));
+    CU(h, cudaMemcpyAsync(h->V, v.data(), (size_t)M * sizeof(float2), cudaMemcpyHostToDevice, h->st));
+    CU(h, cudaMemcpyAsync(h->V + (size_t)N * M, v.data() + 2 * M, (size_t)M * sizeof(float2), cudaMemcpyHostToDevice,
+                          h->st));
     launch_grid_init(h->V, M, N, h->stretch, h->st);
     CHECK_LAUNCH(h);
-    if (iters > 0) {
-      if (!h->V2) CU(h, dalloc(&h->V2, (size_t)M * (N + 1)));
-      CU(h, cudaMemcpyAsync(h->V2, h->V, (size_t)M * (N + 1) * sizeof(float2), cudaMemcpyDeviceToDevice, h->st));
-      float2 *src = h->V, *dst = h->V2;
-      for (int it = 0; it < iters; it++) {
-        launch_grid_jacobi(src, dst, M, N, h->st);
-        std::swap(src, dst);
-      }
-      CHECK_LAUNCH(h);
-      if (src != h->V)
-        CU(h, cudaMemcpyAsync(h->V, src, (size_t)M * (N + 1) * sizeof(float2), cudaMemcpyDeviceToDevice, h->st));
+    // the second buffer: a state buffer that is scratch between steps (M x N x 16 bytes)
+    float2 *src = h->V + M, *dst = reinterpret_cast<float2*>(h->Q[(h->cur + 1) % 3]);
+    for (; done < iters;) {
+      const int k = std::min(iters - done, grid_jacobi_sweeps());
+      launch_grid_jacobi(src, dst, h->V, M, N, k, h->st);
+      std::swap(src, dst);
+      done += k;
     }
+    CHECK_LAUNCH(h);
+    if (src != h->V + M)
+      CU(h, cudaMemcpyAsync(h->V + M, src, (size_t)M * (N - 1) * sizeof(float2), cudaMemcpyDeviceToDevice, h->st));
     launch_f2d(h->V, h->Vd, (size_t)M * (N + 1), h->st);
-    done = iters;
   } else {  // FP64 multicolor Gauss-Seidel from the FP64 boundaries
-    std::vector<double> vd((size_t)M * (N + 1) * 2, 0.0);
-    for (int i = 0; i < M; i++) {
-      vd[2 * i] = h->body[2 * i];
-      vd[2 * i + 1] = h->body[2 * i + 1];
-      size_t o = ((size_t)N * M + i) * 2;
-      vd[o] = h->outer[2 * i];
-      vd[o + 1] = h->outer[2 * i + 1];
-    }
-    CU(h, cudaMemcpyAsync(h->Vd, vd.data(), vd.size() * sizeof(double), cudaMemcpyHostToDevice, h->st));
+    CU(h, cudaMemcpyAsync(h->Vd, h->body.data(), (size_t)M * sizeof(double2), cudaMemcpyHostToDevice, h->st));
+    CU(h, cudaMemcpyAsync(h->Vd + (size_t)N * M, h->outer.data(), (size_t)M * sizeof(double2), cudaMemcpyHostToDevice,
+                          h->st));
     launch_grid_init_d(h->Vd, M, N, h->stretch, h->st);
     CHECK_LAUNCH(h);
-    const int ncol = (M & 1) ? 6 : 4;
     const int check_every = 25;
-    for (int it = 0; it < iters; it++) {
-      CU(h, cudaMemsetAsync(h->move, 0, sizeof(uint32_t), h->st));
-      for (int col = 0; col < ncol; col++) launch_grid_multicolor_d(h->Vd, M, N, col, 1.0, h->move, h->st);
-      done = it + 1;
-      if (tol > 0.0 && (done % check_every == 0 || done == iters)) {
+    double2 *src = h->Vd + M, *dst = reinterpret_cast<double2*>(h->Q[(h->cur + 1) % 3]);
+    while (done < iters) {
+      int k = std::min(iters - done, grid_multicolor_sweeps(M, N));
+      if (tol > 0.0) k = std::min(k, check_every - done % check_every);  // a launch ends at a checked sweep
+      const bool check = tol > 0.0 && ((done + k) % check_every == 0 || done + k == iters);
+      if (check) CU(h, cudaMemsetAsync(h->move, 0, sizeof(uint32_t), h->st));
+      launch_grid_multicolor_d(src, dst, h->Vd, M, N, k, 1.0, check ? h->move : nullptr, h->st);
+      std::swap(src, dst);
+      done += k;
+      if (check) {
         CHECK_LAUNCH(h);
         CU(h, cudaMemcpyAsync(h->h_wave + 1, h->move, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->st));
         CU(h, cudaStreamSynchronize(h->st));
@@ -692,6 +688,8 @@ int ausm_generate_grid(ausm_solver* h, int iters, int method, double tol, int* i
       }
     }
     CHECK_LAUNCH(h);
+    if (src != h->Vd + M)
+      CU(h, cudaMemcpyAsync(h->Vd + M, src, (size_t)M * (N - 1) * sizeof(double2), cudaMemcpyDeviceToDevice, h->st));
     launch_d2f(h->Vd, h->V, (size_t)M * (N + 1), h->st);
   }
   CHECK_LAUNCH(h);

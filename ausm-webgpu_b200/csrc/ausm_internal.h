@@ -234,17 +234,26 @@ void launch_ref_wave(const float4* st, const float4* flen, const float* area, fl
                      uint32_t* wave, cudaStream_t s);
 void launch_dt(const uint32_t* wave, float* dt, float maxdt, float cfl, cudaStream_t s);
 
-// ---- grid, layout, forces, norms (kernels_misc.cu) ----
+// ---- grid generation (kernels_grid.cu) ----
+// V: M x (N + 1) vertices, rows 0 and N given; fills the rows between.
+void launch_grid_init(float2* V, int M, int N, double first_spacing, cudaStream_t s);
+void launch_grid_init_d(double2* V, int M, int N, double first_spacing, cudaStream_t s);
+// `sweeps` elliptic sweeps (at most grid_*_sweeps of them) from src to dst, which hold the
+// rows 1 .. N - 1; rows 0 and N are read from the full vertex array `ends`.  move: max
+// vertex move of the last sweep (float bits, atomicMax), or null.
+int grid_jacobi_sweeps();
+int grid_multicolor_sweeps(int M, int N);
+void launch_grid_jacobi(const float2* src, float2* dst, const float2* ends, int M, int N, int sweeps, cudaStream_t s);
+void launch_grid_multicolor_d(const double2* src, double2* dst, const double2* ends, int M, int N, int sweeps,
+                              double omega, uint32_t* move, cudaStream_t s);
+
+// ---- layout, face records, forces, norms (kernels_misc.cu) ----
 void launch_to_ref_layout(const float4* Qint, float4* ref, const float2* V, const Consts& c, int M, int N,
                           cudaStream_t s);
 void launch_from_ref_layout(const float4* ref, float4* Qint, int M, int N, cudaStream_t s);
 void launch_fill(float4* Q, float4 v, size_t n, cudaStream_t s);
-void launch_grid_init(float2* V, int M, int N, double first_spacing, cudaStream_t s);
-void launch_grid_jacobi(const float2* src, float2* dst, int M, int N, cudaStream_t s);
 // parts: 2 * kMaxParts doubles of scratch; acc gets the sums, in a fixed order.
-// FP64 grid and face records (kernels_misc.cu): see k_metrics_d for the record layout.
-void launch_grid_init_d(double2* V, int M, int N, double first_spacing, cudaStream_t s);
-void launch_grid_multicolor_d(double2* V, int M, int N, int color, double omega, uint32_t* move, cudaStream_t s);
+// FP64 face records: see k_metrics_d for their layout.
 void launch_d2f(const double2* a, float2* b, size_t n, cudaStream_t s);
 void launch_f2d(const float2* a, double2* b, size_t n, cudaStream_t s);
 void launch_metrics_d(const double2* V, float4* Mi, float4* Mj, int M, int N, cudaStream_t s);

@@ -1,4 +1,4 @@
-// Grid generation, layout conversion, surface forces, residual norms and field output.
+// Vertex and layout conversion, face records, surface forces, residual norms and field output.
 #include "ausm_internal.h"
 
 namespace ausm {
@@ -29,116 +29,7 @@ __global__ void k_fill(float4* __restrict__ Q, float4 v, size_t n) {
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) Q[k] = v;
 }
 
-// ---- grid ----
-// Initial guess (shaders/grid.js:18-27): mix(body, outer, t) along each i line,
-// t = j/N (reference) or a geometric progression with first cell height `h1` relative
-// to the body-outer distance of that line.
-__global__ void k_grid_init(float2* __restrict__ V, int M, int N, double first_spacing) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= M || j > N || j == 0 || j == N) return;
-  float2 a = V[i], b = V[(size_t)N * M + i];
-  float t;
-  if (first_spacing <= 0.0) {
-    t = float(j) / float(N);
-  } else {
-    double L = sqrt((double)(b.x - a.x) * (b.x - a.x) + (double)(b.y - a.y) * (b.y - a.y));
-    double h = first_spacing / L;  // first step as a fraction of the line length
-    // growth ratio q solves h (q^N - 1)/(q - 1) = 1 (bisection, fixed iteration count)
-    double lo = 1.0 + 1e-12, hi = 2.0;
-    if (h * N >= 1.0) { lo = 1e-6; hi = 1.0 - 1e-12; }
-    for (int it = 0; it < 200; it++) {
-      double q = 0.5 * (lo + hi);
-      double s = h * (pow(q, (double)N) - 1.0) / (q - 1.0);
-      if ((s > 1.0) == (h * N < 1.0)) hi = q; else lo = q;
-    }
-    double q = 0.5 * (lo + hi);
-    t = (float)(h * (pow(q, (double)j) - 1.0) / (q - 1.0));
-  }
-  V[(size_t)j * M + i] = make_float2(a.x * (1.0f - t) + b.x * t, a.y * (1.0f - t) + b.y * t);
-}
-
-// TTM/Winslow update with P = Q = 0, omega = 1, applied only where the Jacobian is
-// negative (shaders/grid.js:55-108); i wraps through the seam.
-__device__ __forceinline__ float2 ttm_point(const float2* __restrict__ s, int M, int i, int j, float omega) {
-  int l = i == 0 ? M - 1 : i - 1, r = i == M - 1 ? 0 : i + 1;
-  size_t rj = (size_t)j * M, ru = (size_t)(j + 1) * M, rd = (size_t)(j - 1) * M;
-  float2 c = s[rj + i], L = s[rj + l], R = s[rj + r], D = s[rd + i], U = s[ru + i];
-  float2 DL = s[rd + l], DR = s[rd + r], UL = s[ru + l], UR = s[ru + r];
-  float xix = 0.5f * (R.x - L.x), xiy = 0.5f * (R.y - L.y);
-  float etx = 0.5f * (U.x - D.x), ety = 0.5f * (U.y - D.y);
-  float xex = 0.25f * (UR.x + DL.x - UL.x - DR.x), xey = 0.25f * (UR.y + DL.y - UL.y - DR.y);
-  float alpha = etx * etx + ety * ety, gam = xix * xix + xiy * xiy, beta = xix * etx + xiy * ety;
-  const float Pc = 0.0f, Qc = 0.0f;
-  float den = 2.0f * (alpha + gam);
-  float npx = (alpha * (L.x + R.x + Pc * xix) + gam * (D.x + U.x + Qc * etx) - 2.0f * beta * xex) / den;
-  float npy = (alpha * (L.y + R.y + Pc * xiy) + gam * (D.y + U.y + Qc * ety) - 2.0f * beta * xey) / den;
-  float jac = xix * ety - xiy * etx;
-  if (jac < 0.0f) return make_float2(c.x * (1.0f - omega) + npx * omega, c.y * (1.0f - omega) + npy * omega);
-  return c;
-}
-__global__ void k_grid_jacobi(const float2* __restrict__ src, float2* __restrict__ dst, int M, int N) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= M || j < 1 || j >= N) return;
-  dst[(size_t)j * M + i] = ttm_point(src, M, i, j, 1.0f);
-}
-
-// ---- FP64 grid (multicolor TTM generator of the fused engine) and FP64 metrics ----
-__global__ void k_grid_init_d(double2* __restrict__ V, int M, int N, double first_spacing) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= M || j > N || j == 0 || j == N) return;
-  double2 a = V[i], b = V[(size_t)N * M + i];
-  double t;
-  if (first_spacing <= 0.0) {
-    t = (double)j / (double)N;
-  } else {
-    double L = sqrt((b.x - a.x) * (b.x - a.x) + (b.y - a.y) * (b.y - a.y));
-    double h = first_spacing / L;
-    double lo = 1.0 + 1e-12, hi = 2.0;
-    if (h * N >= 1.0) { lo = 1e-6; hi = 1.0 - 1e-12; }
-    for (int it = 0; it < 200; it++) {
-      double q = 0.5 * (lo + hi);
-      double s = h * (pow(q, (double)N) - 1.0) / (q - 1.0);
-      if ((s > 1.0) == (h * N < 1.0)) hi = q; else lo = q;
-    }
-    double q = 0.5 * (lo + hi);
-    t = h * (pow(q, (double)j) - 1.0) / (q - 1.0);
-  }
-  V[(size_t)j * M + i] = make_double2(a.x * (1.0 - t) + b.x * t, a.y * (1.0 - t) + b.y * t);
-}
-
-__device__ __forceinline__ double2 ttm_point_d(const double2* __restrict__ s, int M, int i, int j, double omega) {
-  int l = i == 0 ? M - 1 : i - 1, r = i == M - 1 ? 0 : i + 1;
-  size_t rj = (size_t)j * M, ru = (size_t)(j + 1) * M, rd = (size_t)(j - 1) * M;
-  double2 c = s[rj + i], L = s[rj + l], R = s[rj + r], D = s[rd + i], U = s[ru + i];
-  double2 DL = s[rd + l], DR = s[rd + r], UL = s[ru + l], UR = s[ru + r];
-  double xix = 0.5 * (R.x - L.x), xiy = 0.5 * (R.y - L.y);
-  double etx = 0.5 * (U.x - D.x), ety = 0.5 * (U.y - D.y);
-  double xex = 0.25 * (UR.x + DL.x - UL.x - DR.x), xey = 0.25 * (UR.y + DL.y - UL.y - DR.y);
-  double alpha = etx * etx + ety * ety, gam = xix * xix + xiy * xiy, beta = xix * etx + xiy * ety;
-  double den = 2.0 * (alpha + gam);
-  double npx = (alpha * (L.x + R.x) + gam * (D.x + U.x) - 2.0 * beta * xex) / den;
-  double npy = (alpha * (L.y + R.y) + gam * (D.y + U.y) - 2.0 * beta * xey) / den;
-  double jac = xix * ety - xiy * etx;
-  if (jac < 0.0) return make_double2(c.x * (1.0 - omega) + npx * omega, c.y * (1.0 - omega) + npy * omega);
-  return c;
-}
-// One colour of the FP64 multicolour Gauss-Seidel sweep: colour (i&1)*2 + (j&1); with odd
-// M the seam column i = M-1 is coloured 4 + (j&1) so no two points of a colour touch
-// (9-point stencil, periodic in i).  Records the max vertex move (float bits).
-__global__ void k_grid_multicolor_d(double2* __restrict__ V, int M, int N, int color, double omega, uint32_t* move) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-  uint32_t mv = 0u;
-  if (i < M && j >= 1 && j < N) {
-    int col = ((M & 1) && i == M - 1) ? 4 + (j & 1) : (i & 1) * 2 + (j & 1);
-    if (col == color) {
-      double2 p = ttm_point_d(V, M, i, j, omega);
-      double2 o = V[(size_t)j * M + i];
-      mv = __float_as_uint((float)fmax(fabs(p.x - o.x), fabs(p.y - o.y)));
-      V[(size_t)j * M + i] = p;
-    }
-  }
-  block_max_to(move, mv);
-}
+// ---- vertex conversion and FP64 metrics ----
 __global__ void k_d2f(const double2* __restrict__ a, float2* __restrict__ b, size_t n) {
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
     b[k] = make_float2((float)a[k].x, (float)a[k].y);
@@ -271,12 +162,6 @@ void launch_from_ref_layout(const float4* ref, float4* Qint, int M, int N, cudaS
   k_from_ref_layout<<<grid1d(n), 256, 0, s>>>(ref, Qint, n, M);
 }
 void launch_fill(float4* Q, float4 v, size_t n, cudaStream_t s) { k_fill<<<grid1d(n), 256, 0, s>>>(Q, v, n); }
-void launch_grid_init(float2* V, int M, int N, double first_spacing, cudaStream_t s) {
-  k_grid_init<<<grid16(M, N + 1), B16, 0, s>>>(V, M, N, first_spacing);
-}
-void launch_grid_jacobi(const float2* src, float2* dst, int M, int N, cudaStream_t s) {
-  k_grid_jacobi<<<grid16(M, N + 1), B16, 0, s>>>(src, dst, M, N);
-}
 void launch_forces(const float4* row0, const double2* V, const Consts& c, int M, double* acc, double* parts,
                    double* cp, double q_inf, double p_inf, cudaStream_t s) {
   int blocks = std::min((M + 255) / 256, 148);
@@ -287,12 +172,6 @@ void launch_sumsq_rho(const float4* R, size_t n, double* acc, double* parts, cud
   const int blocks = grid1d(n);  // <= kMaxParts
   k_sumsq_rho<<<blocks, 256, 0, s>>>(R, n, parts);
   k_sum_parts<<<1, 256, 0, s>>>(parts, blocks, acc);
-}
-void launch_grid_init_d(double2* V, int M, int N, double first_spacing, cudaStream_t s) {
-  k_grid_init_d<<<grid16(M, N + 1), B16, 0, s>>>(V, M, N, first_spacing);
-}
-void launch_grid_multicolor_d(double2* V, int M, int N, int color, double omega, uint32_t* move, cudaStream_t s) {
-  k_grid_multicolor_d<<<grid16(M, N + 1), B16, 0, s>>>(V, M, N, color, omega, move);
 }
 void launch_d2f(const double2* a, float2* b, size_t n, cudaStream_t s) { k_d2f<<<grid1d(n), 256, 0, s>>>(a, b, n); }
 void launch_f2d(const float2* a, double2* b, size_t n, cudaStream_t s) { k_f2d<<<grid1d(n), 256, 0, s>>>(a, b, n); }

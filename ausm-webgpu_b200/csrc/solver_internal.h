@@ -22,7 +22,6 @@ struct ausm_solver {
   bool has_body = false, has_outer = false, has_grid = false, has_state = false;
   double stretch = 0.0;
   float2* V = nullptr;    // vertices, FP32 (reference layout, API, reference engine)
-  float2* V2 = nullptr;   // Jacobi ping-pong
   double2* Vd = nullptr;  // vertices, FP64 (multicolor generator, metrics, forces)
   float4* Mi = nullptr;   // FP64-computed face records, i-faces [N][M]
   float4* Mj = nullptr;   // ... j-faces [N+1][M]
