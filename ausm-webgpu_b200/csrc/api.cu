@@ -893,21 +893,15 @@ int step_impl(ausm_solver* h, int n, float* dt_out, bool read_err) {
         h->cur = b;
       }
     } else {
-      // texture ping-pong of main.js:744-777
+      // main.js:744-777 without the copies of its texture ping-pong
       float4 **S = h->S;
       for (int k = 0; k < n; k++) {
-        launch_ref_boundary(S[2], S[0], h->V, h->c, M, N, s);
-        launch_ref_fluxes(sch, S[0], h->V, h->fx, h->fy, h->c, M, N, s);
-        launch_ref_residual(h->fx, h->fy, h->flen, h->area, h->res, M, N, s);
-        launch_ref_rk(1, h->res, S[0], nullptr, S[1], h->dt, M, N, s);
-        launch_ref_boundary(S[1], S[2], h->V, h->c, M, N, s);
         launch_ref_fluxes(sch, S[2], h->V, h->fx, h->fy, h->c, M, N, s);
-        launch_ref_residual(h->fx, h->fy, h->flen, h->area, h->res, M, N, s);
-        launch_ref_rk(2, h->res, S[0], S[1], S[2], h->dt, M, N, s);
-        launch_ref_boundary(S[2], S[1], h->V, h->c, M, N, s);
+        launch_ref_stage(1, h->fx, h->fy, h->flen, h->area, S[2], nullptr, S[1], h->dt, M, N, s);
         launch_ref_fluxes(sch, S[1], h->V, h->fx, h->fy, h->c, M, N, s);
-        launch_ref_residual(h->fx, h->fy, h->flen, h->area, h->res, M, N, s);
-        launch_ref_rk(3, h->res, S[0], S[1], S[2], h->dt, M, N, s);
+        launch_ref_stage(2, h->fx, h->fy, h->flen, h->area, S[2], S[1], S[0], h->dt, M, N, s);
+        launch_ref_fluxes(sch, S[0], h->V, h->fx, h->fy, h->c, M, N, s);
+        launch_ref_stage(3, h->fx, h->fy, h->flen, h->area, S[2], S[0], S[2], h->dt, M, N, s);
       }
       launch_ref_wave(S[2], h->flen, h->area, h->c.gamma, M, N, h->wave, s);
     }
@@ -998,8 +992,7 @@ int ausm_residual_l2(ausm_solver* h, double* l2) {
                        N, nullptr, 16, h->err_flag, h->st);
     R = scratch;
   } else {
-    launch_ref_boundary(h->S[2], h->S[0], h->V, h->c, M, N, h->st);
-    launch_ref_fluxes(h->p.scheme, h->S[0], h->V, h->fx, h->fy, h->c, M, N, h->st);
+    launch_ref_fluxes(h->p.scheme, h->S[2], h->V, h->fx, h->fy, h->c, M, N, h->st);
     launch_ref_residual(h->fx, h->fy, h->flen, h->area, h->res, M, N, h->st);
     R = h->res;
   }

@@ -228,8 +228,8 @@ void launch_ref_fluxes(int scheme, const float4* st, const float2* V, float4* fx
                        int N, cudaStream_t s);
 void launch_ref_residual(const float4* fx, const float4* fy, const float4* flen, const float* area, float4* res, int M,
                          int N, cudaStream_t s);
-void launch_ref_rk(int stage, const float4* res, const float4* s0, const float4* s1, float4* out, const float* dt,
-                   int M, int N, cudaStream_t s);
+void launch_ref_stage(int stage, const float4* fx, const float4* fy, const float4* flen, const float* area,
+                      const float4* s0, const float4* s1, float4* out, const float* dt, int M, int N, cudaStream_t s);
 void launch_ref_wave(const float4* st, const float4* flen, const float* area, float gamma, int M, int N,
                      uint32_t* wave, cudaStream_t s);
 void launch_dt(const uint32_t* wave, float* dt, float maxdt, float cfl, cudaStream_t s);

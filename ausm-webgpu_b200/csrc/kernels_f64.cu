@@ -1,5 +1,5 @@
-// Full-FP64 engine: the reference's dispatch structure (boundary, j-flux, i-flux,
-// residual, RK stage per stage; wave-speed max once per step(n) call, main.js:744-791)
+// Full-FP64 engine: the reference's operators (boundary, j- and i-flux; residual and RK
+// stage: two kernels a stage; wave-speed max once per step(n) call, main.js:744-791)
 // on FP64 buffers, with FP64 metrics from the FP64 vertices and every operation in
 // double (physics_exact.cuh; compiled with -fmad=false).  It exists to state the FP32
 // engines' error against an FP64 solution of the same problem on the same grid.
@@ -7,8 +7,13 @@
 // Layout as the reference engine, in double: state double4 [N+3][M] (row 0 wall ghost,
 // rows N+1, N+2 far field), fluxes double4 [N][M] (i) and [N+1][M] (j), residual
 // double4 [N][M], face lengths double4 and cell areas double [N][M].
+//
+// Bound by FP64 arithmetic in the flux kernel: two faces a cell with some 28 divisions and
+// square roots each, about 700 operations, 31 us a stage of 512 x 384.  With one kernel per
+// dispatch a pass of 10 steps and the state's read-back took 2.4 ms, now 1.8.
 #include "ausm_internal.h"
 #include "physics_exact.cuh"
+#include "tma.cuh"
 
 namespace ausm {
 
@@ -19,10 +24,17 @@ using R = double;
 
 namespace {
 
-__device__ __forceinline__ V4<R> ld(const V4<R>* st, int M, int i, int j) {  // loadState, ausm.js:138-143
-  int ii = (i + M) % M;
-  int jj = max(j + 1, 0);
-  return st[(size_t)jj * M + ii];
+// State of cell (i, j), j in [-2, N + 1], from interior rows alone: loadState (ausm.js:138-143;
+// i wraps, interior row + 1, clamped at the wall ghost) with the ghost rows of the boundary
+// pass (ausm.js:23-120) computed where they are read.
+__device__ __forceinline__ V4<R> ld(const V4<R>* st, const V2<R>* V, const ConstsR<R>& c, int M, int N, int i, int j) {
+  const int ii = (i + M) % M, jj = max(j + 1, 0);
+  if (jj >= 1 && jj <= N) return st[(size_t)jj * M + ii];
+  const int r = (ii + 1) % M;
+  if (jj == 0) return ex::wall_ghost(st[(size_t)M + ii], V[ii], V[r]);
+  V4<R> g1, g2;
+  ex::far_ghosts(st[(size_t)N * M + ii], V[(size_t)N * M + ii], V[(size_t)N * M + r], c, g1, g2);
+  return jj == N + 1 ? g1 : g2;
 }
 
 __global__ void k_ex_metrics(const V2<R>* __restrict__ V, R* __restrict__ area, V4<R>* __restrict__ flen, int M,
@@ -45,6 +57,8 @@ __global__ void k_ex_boundary(const V4<R>* __restrict__ in, V4<R>* __restrict__ 
   int i = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= M || y >= N + 3) return;
   int r = (i + 1) % M;
+  grid_dep_wait();
+  grid_dep_launch();
   if (y == 0) {
     out[i] = ex::wall_ghost(in[(size_t)M + i], V[i], V[r]);
   } else if (y > N) {
@@ -56,55 +70,73 @@ __global__ void k_ex_boundary(const V4<R>* __restrict__ in, V4<R>* __restrict__ 
   }
 }
 
+// The j- and i-flux passes: a block converts the cells of its 32 x 8 faces (with the three
+// rows and columns beside them) to primitives once, in shared memory, and its threads take
+// one face of each direction.  Two kernels that converted the four cells of every face
+// spent a quarter of their time on that (8 conversions per cell, two divisions each).
 template <int SCHEME>
-__global__ void k_ex_flux_j(const V4<R>* __restrict__ st, const V2<R>* __restrict__ V, V4<R>* __restrict__ fy,
-                            const ConstsR<R> c, int M, int N) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= M || j > N) return;
-  R nx, ny, len;
-  ex::edge_normal(V[(size_t)j * M + i], V[(size_t)j * M + (i + 1) % M], nx, ny, len);
-  fy[(size_t)j * M + i] = ex::face_flux<SCHEME>(ex::to_prim(ld(st, M, i, j - 2), c.gm1),
-                                                ex::to_prim(ld(st, M, i, j - 1), c.gm1),
-                                                ex::to_prim(ld(st, M, i, j), c.gm1),
-                                                ex::to_prim(ld(st, M, i, j + 1), c.gm1), nx, ny, c);
+__global__ void __launch_bounds__(256)
+    k_ex_fluxes(const V4<R>* __restrict__ st, const V2<R>* __restrict__ V, V4<R>* __restrict__ fx,
+                 V4<R>* __restrict__ fy, const ConstsR<R> c, int M, int N) {
+  __shared__ V4<R> P[11][35];
+  const int tx = threadIdx.x, ty = threadIdx.y, i0 = blockIdx.x * 32, j0 = blockIdx.y * 8;
+  const int i = i0 + tx, j = j0 + ty;
+  const bool jf = i < M && j <= N, jn = i < M && j < N;
+  R nx = 0, ny = 0, mx = 0, my = 0, len;
+  if (jf) ex::edge_normal(V[(size_t)j * M + i], V[(size_t)j * M + (i + 1) % M], nx, ny, len);
+  if (jn) ex::edge_normal(V[(size_t)(j + 1) * M + i], V[(size_t)j * M + i], mx, my, len);
+  grid_dep_wait();
+  grid_dep_launch();
+  for (int k = ty * 32 + tx; k < 11 * 35; k += 256) {
+    const int r = k / 35, cc = k % 35;
+    if (j0 - 2 + r <= N + 1 && i0 - 2 + cc <= M)
+      P[r][cc] = ex::to_prim(ld(st, V, c, M, N, i0 - 2 + cc, j0 - 2 + r), c.gm1);
+  }
+  __syncthreads();
+  if (jf)
+    fy[(size_t)j * M + i] = ex::face_flux<SCHEME>(P[ty][tx + 2], P[ty + 1][tx + 2], P[ty + 2][tx + 2], P[ty + 3][tx + 2], nx, ny, c);
+  if (jn)
+    fx[(size_t)j * M + i] = ex::face_flux<SCHEME>(P[ty + 2][tx], P[ty + 2][tx + 1], P[ty + 2][tx + 2], P[ty + 2][tx + 3], mx, my, c);
 }
 
-template <int SCHEME>
-__global__ void k_ex_flux_i(const V4<R>* __restrict__ st, const V2<R>* __restrict__ V, V4<R>* __restrict__ fx,
-                            const ConstsR<R> c, int M, int N) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= M || j >= N) return;
-  R nx, ny, len;
-  ex::edge_normal(V[(size_t)(j + 1) * M + i], V[(size_t)j * M + i], nx, ny, len);
-  fx[(size_t)j * M + i] = ex::face_flux<SCHEME>(ex::to_prim(ld(st, M, i - 2, j), c.gm1),
-                                                ex::to_prim(ld(st, M, i - 1, j), c.gm1),
-                                                ex::to_prim(ld(st, M, i, j), c.gm1),
-                                                ex::to_prim(ld(st, M, i + 1, j), c.gm1), nx, ny, c);
-}
-
-__global__ void k_ex_residual(const V4<R>* __restrict__ fx, const V4<R>* __restrict__ fy,
-                              const V4<R>* __restrict__ flen, const R* __restrict__ area, V4<R>* __restrict__ res,
-                              int M, int N) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= M || j >= N) return;
+// residual of a cell from its faces (ausm.js:402-436)
+__device__ __forceinline__ V4<R> residual_of(const V4<R>* __restrict__ fx, const V4<R>* __restrict__ fy,
+                                             const V4<R>* __restrict__ flen, const R* __restrict__ area, int M, int i,
+                                             int j) {
   size_t k = (size_t)j * M + i;
   V4<R> xl = fx[k], xr = fx[(size_t)j * M + (i + 1) % M], yu = fy[(size_t)(j + 1) * M + i], yd = fy[k];
   V4<R> l = flen[k];
   R A = area[k];
-  res[k] = {-(xr.x * l.y - xl.x * l.x + yu.x * l.z - yd.x * l.w) / A,
-            -(xr.y * l.y - xl.y * l.x + yu.y * l.z - yd.y * l.w) / A,
-            -(xr.z * l.y - xl.z * l.x + yu.z * l.z - yd.z * l.w) / A,
-            -(xr.w * l.y - xl.w * l.x + yu.w * l.z - yd.w * l.w) / A};
+  return {-(xr.x * l.y - xl.x * l.x + yu.x * l.z - yd.x * l.w) / A,
+          -(xr.y * l.y - xl.y * l.x + yu.y * l.z - yd.y * l.w) / A,
+          -(xr.z * l.y - xl.z * l.x + yu.z * l.z - yd.z * l.w) / A,
+          -(xr.w * l.y - xl.w * l.x + yu.w * l.z - yd.w * l.w) / A};
 }
-
-template <int STAGE>
-__global__ void k_ex_rk(const V4<R>* __restrict__ res, const V4<R>* __restrict__ s0, const V4<R>* __restrict__ s1,
-                        V4<R>* __restrict__ out, const R* __restrict__ dtp, int M, int N) {
+__global__ void k_ex_residual(const V4<R>* __restrict__ fx, const V4<R>* __restrict__ fy,
+                               const V4<R>* __restrict__ flen, const R* __restrict__ area,
+                               V4<R>* __restrict__ res, int M, int N) {
   int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= M || j >= N) return;
+  grid_dep_wait();
+  grid_dep_launch();
+  res[(size_t)j * M + i] = residual_of(fx, fy, flen, area, M, i, j);
+}
+
+// residual and RK stage (ausm.js:402-527) of the interior rows; the residual, which only
+// this stage uses, stays in registers
+template <int STAGE>
+__global__ void k_ex_stage(const V4<R>* __restrict__ fx, const V4<R>* __restrict__ fy,
+                            const V4<R>* __restrict__ flen, const R* __restrict__ area, const V4<R>* s0,
+                            const V4<R>* __restrict__ s1, V4<R>* out, const R* __restrict__ dtp, int M,
+                            int N) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+  if (i >= M || j >= N) return;
+  grid_dep_wait();
+  grid_dep_launch();
   const R dt = *dtp;
-  size_t k = (size_t)j * M + i, o = (size_t)(j + 1) * M + i;
-  V4<R> Rr = res[k], Q = s0[o], o4;
+  size_t o = (size_t)(j + 1) * M + i;
+  const V4<R> Rr = residual_of(fx, fy, flen, area, M, i, j), Q = s0[o];
+  V4<R> o4;
   if constexpr (STAGE == 1) {
     o4 = {Q.x + dt * Rr.x, Q.y + dt * Rr.y, Q.z + dt * Rr.z, Q.w + dt * Rr.w};
   } else if constexpr (STAGE == 2) {
@@ -122,6 +154,8 @@ __global__ void k_ex_rk(const V4<R>* __restrict__ res, const V4<R>* __restrict__
 // max of the FP64 wave speed: positive doubles order like their bit patterns
 __global__ void k_ex_wave(const V4<R>* __restrict__ st, const V4<R>* __restrict__ flen, const R* __restrict__ area,
                           R gamma, int M, int N, unsigned long long* wave) {
+  grid_dep_wait();
+  grid_dep_launch();
   __shared__ unsigned long long red[8];
   unsigned long long wm = 0ull;
   size_t total = (size_t)M * N;
@@ -195,8 +229,7 @@ inline int grid1d(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 148 
 template <int SCHEME>
 void fluxes(const V4<R>* st, const V2<R>* V, V4<R>* fx, V4<R>* fy, const ConstsR<R>& c, int M, int N,
             cudaStream_t s) {
-  k_ex_flux_j<SCHEME><<<grid16(M, N + 1), B16, 0, s>>>(st, V, fy, c, M, N);
-  k_ex_flux_i<SCHEME><<<grid16(M, N), B16, 0, s>>>(st, V, fx, c, M, N);
+  launch_pdl(k_ex_fluxes<SCHEME>, dim3((M + 31) / 32, (N + 8) / 8), dim3(32, 8), 0, s, st, V, fx, fy, c, M, N);
 }
 
 }  // namespace
@@ -233,7 +266,7 @@ void F64Engine::from_f32(const float4* ref, cudaStream_t s) {
 }
 void F64Engine::to_f32(float4* ref, const double2* Vd, cudaStream_t s) {
   // boundary pass into S[0] (the reference layout with its ghost rows), then rounded
-  k_ex_boundary<<<grid16(M, N + 3), B16, 0, s>>>(S[2], S[0], reinterpret_cast<const V2<R>*>(Vd), c, M, N);
+  launch_pdl(k_ex_boundary, grid16(M, N + 3), B16, 0, s, S[2], S[0], reinterpret_cast<const V2<R>*>(Vd), c, M, N);
   const size_t n = (size_t)M * (N + 3);
   k_ex_to_f32<<<grid1d(n), 256, 0, s>>>(S[0], ref, n);
 }
@@ -242,13 +275,13 @@ void F64Engine::fill(double rho, double ru, double rv, double E, cudaStream_t s)
   k_ex_fill<<<grid1d(n), 256, 0, s>>>(S[2], V4<R>{rho, ru, rv, E}, n);
 }
 const void* F64Engine::state_ref(const double2* Vd, cudaStream_t s) {
-  k_ex_boundary<<<grid16(M, N + 3), B16, 0, s>>>(S[2], S[0], reinterpret_cast<const V2<R>*>(Vd), c, M, N);
+  launch_pdl(k_ex_boundary, grid16(M, N + 3), B16, 0, s, S[2], S[0], reinterpret_cast<const V2<R>*>(Vd), c, M, N);
   return S[0];
 }
 void F64Engine::wave_speed(cudaStream_t s) {
   cudaMemsetAsync(wave, 0, sizeof(unsigned long long), s);
   int blocks = (int)std::min<size_t>(((size_t)M * N + 255) / 256, 148 * 8);
-  k_ex_wave<<<blocks, 256, 0, s>>>(S[2], flen, area, c.gamma, M, N, wave);
+  launch_pdl(k_ex_wave, dim3(blocks), dim3(256), 0, s, S[2], flen, area, c.gamma, M, N, wave);
 }
 void F64Engine::step(int scheme, int n, const double2* Vd_, cudaStream_t s) {
   const V2<R>* Vd = reinterpret_cast<const V2<R>*>(Vd_);
@@ -257,29 +290,24 @@ void F64Engine::step(int scheme, int n, const double2* Vd_, cudaStream_t s) {
     if (scheme == 0) fluxes<0>(st, Vd, fx, fy, c, M, N, s);
     else if (scheme == 1) fluxes<1>(st, Vd, fx, fy, c, M, N, s);
     else fluxes<2>(st, Vd, fx, fy, c, M, N, s);
-    k_ex_residual<<<grid16(M, N), B16, 0, s>>>(fx, fy, flen, area, res, M, N);
   };
-  const dim3 gb = grid16(M, N + 3), gi = grid16(M, N);
-  for (int k = 0; k < n; k++) {  // the texture ping-pong of main.js:744-777
-    k_ex_boundary<<<gb, B16, 0, s>>>(S[2], S[0], Vd, c, M, N);
-    flux(S[0]);
-    k_ex_rk<1><<<gi, B16, 0, s>>>(res, S[0], nullptr, S[1], dt, M, N);
-    k_ex_boundary<<<gb, B16, 0, s>>>(S[1], S[2], Vd, c, M, N);
+  const dim3 gi = grid16(M, N);
+  for (int k = 0; k < n; k++) {  // main.js:744-777 without the copies of its texture ping-pong
     flux(S[2]);
-    k_ex_rk<2><<<gi, B16, 0, s>>>(res, S[0], S[1], S[2], dt, M, N);
-    k_ex_boundary<<<gb, B16, 0, s>>>(S[2], S[1], Vd, c, M, N);
+    launch_pdl(k_ex_stage<1>, gi, B16, 0, s, fx, fy, flen, area, S[2], nullptr, S[1], dt, M, N);
     flux(S[1]);
-    k_ex_rk<3><<<gi, B16, 0, s>>>(res, S[0], S[1], S[2], dt, M, N);
+    launch_pdl(k_ex_stage<2>, gi, B16, 0, s, fx, fy, flen, area, S[2], S[1], S[0], dt, M, N);
+    flux(S[0]);
+    launch_pdl(k_ex_stage<3>, gi, B16, 0, s, fx, fy, flen, area, S[2], S[0], S[2], dt, M, N);
   }
   if (n > 0) wave_speed(s);
 }
 void F64Engine::residual(int scheme, const double2* Vd_, cudaStream_t s) {
   const V2<R>* Vd = reinterpret_cast<const V2<R>*>(Vd_);
-  k_ex_boundary<<<grid16(M, N + 3), B16, 0, s>>>(S[2], S[0], Vd, c, M, N);
-  if (scheme == 0) fluxes<0>(S[0], Vd, fx, fy, c, M, N, s);
-  else if (scheme == 1) fluxes<1>(S[0], Vd, fx, fy, c, M, N, s);
-  else fluxes<2>(S[0], Vd, fx, fy, c, M, N, s);
-  k_ex_residual<<<grid16(M, N), B16, 0, s>>>(fx, fy, flen, area, res, M, N);
+  if (scheme == 0) fluxes<0>(S[2], Vd, fx, fy, c, M, N, s);
+  else if (scheme == 1) fluxes<1>(S[2], Vd, fx, fy, c, M, N, s);
+  else fluxes<2>(S[2], Vd, fx, fy, c, M, N, s);
+  launch_pdl(k_ex_residual, grid16(M, N), B16, 0, s, fx, fy, flen, area, res, M, N);
 }
 void F64Engine::sumsq_rho(double* parts, double* acc, cudaStream_t s) {
   const size_t n = (size_t)M * N;

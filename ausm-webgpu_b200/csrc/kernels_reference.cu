@@ -1,5 +1,6 @@
-// Reference-shaped engine: the reference's five dispatches per RK stage, one CUDA
-// kernel each, on the reference's buffer layout (main.js:110-125):
+// Reference-shaped engine: the reference's five dispatches per RK stage as two CUDA
+// kernels (boundary, j- and i-flux; residual and RK stage), fluxes and states going through
+// memory, on the reference's buffer layout (main.js:110-125):
 //   boundary  ausm.js:23-120   M x (N+3)   ghost rows + pass-through copy
 //   j-flux    ausm.js:128-392  M x (N+1)   faces below each interior cell
 //   i-flux    ausm.js:128-392  M x N       faces left of each interior cell (the
@@ -10,16 +11,27 @@
 // plus the wave-speed max reduction (ausm.js:617-630, 535-581) and the grid metrics
 // (shaders/grid.js:115-147).  This translation unit is compiled with -fmad=false and
 // uses the exact (FAST=false) arithmetic, so it matches the float oracle bit for bit.
-// It is the plain one-launch-per-dispatch baseline of the benchmarks.
+// It is the plain baseline of the benchmarks.
+// Bound by its IEEE divisions and square roots (some 50 a cell and stage) and by latency.  A
+// step of 510 x 381 (AUSM+-up) took 100 us with one kernel per dispatch (full copies in the
+// boundary pass, the residual through memory, eight conversions to primitives per cell),
+// 75 us with those kernels under programmatic dependent launch, and takes 52 us.
 #include "ausm_internal.h"
+#include "tma.cuh"
 
 namespace ausm {
 
-__device__ __forceinline__ float4 ref_load(const float4* __restrict__ st, int M, int i, int j) {
-  // loadState (ausm.js:138-143): i wraps, interior index + 1, clamped at the wall ghost
-  int ii = (i + M) % M;
-  int jj = max(j + 1, 0);
-  return st[(size_t)jj * M + ii];
+// State of cell (i, j), j in [-2, N + 1], from interior rows alone: loadState (ausm.js:138-143;
+// i wraps, interior row + 1, clamped at the wall ghost) with the ghost rows of the boundary
+// pass (ausm.js:23-120) computed where they are read.
+__device__ __forceinline__ float4 ref_load(const float4* st, const float2* V, const Consts& c, int M, int N, int i, int j) {
+  const int ii = (i + M) % M, jj = max(j + 1, 0);
+  if (jj >= 1 && jj <= N) return st[(size_t)jj * M + ii];
+  const int r = (ii + 1) % M;
+  if (jj == 0) return wall_ghost<false>(st[(size_t)M + ii], V[ii], V[r]);
+  float4 g1, g2;
+  far_ghosts<false>(st[(size_t)N * M + ii], V[(size_t)N * M + ii], V[(size_t)N * M + r], c, g1, g2);
+  return jj == N + 1 ? g1 : g2;
 }
 
 __global__ void k_ref_metrics(const float2* __restrict__ V, float* __restrict__ area, float4* __restrict__ flen,
@@ -44,6 +56,8 @@ __global__ void k_ref_boundary(const float4* __restrict__ in, float4* __restrict
   int i = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= M || y >= N + 3) return;
   int r = (i + 1) % M;
+  grid_dep_wait();
+  grid_dep_launch();
   if (y == 0) {
     out[i] = wall_ghost<false>(in[(size_t)M + i], V[i], V[r]);
   } else if (y > N) {
@@ -55,41 +69,39 @@ __global__ void k_ref_boundary(const float4* __restrict__ in, float4* __restrict
   }
 }
 
+// The j- and i-flux passes: a block converts the cells of its 32 x 8 faces (with the three
+// rows and columns beside them) to primitives once, in shared memory, and its threads take
+// one face of each direction.  Two kernels that converted the four cells of every face
+// spent a quarter of their time on that (8 conversions per cell, two divisions each).
 template <int SCHEME>
-__global__ void k_ref_flux_j(const float4* __restrict__ st, const float2* __restrict__ V, float4* __restrict__ fy,
-                             const Consts c, int M, int N) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= M || j > N) return;
-  float nx, ny, len;
-  edge_normal<false>(V[(size_t)j * M + i], V[(size_t)j * M + (i + 1) % M], nx, ny, len);
-  const float gm1 = c.gm1;
-  float4 f = face_flux<SCHEME>(to_prim<false>(ref_load(st, M, i, j - 2), gm1),
-                                      to_prim<false>(ref_load(st, M, i, j - 1), gm1),
-                                      to_prim<false>(ref_load(st, M, i, j), gm1),
-                                      to_prim<false>(ref_load(st, M, i, j + 1), gm1), nx, ny, c);
-  fy[(size_t)j * M + i] = f;
+__global__ void __launch_bounds__(256)
+    k_ref_fluxes(const float4* __restrict__ st, const float2* __restrict__ V, float4* __restrict__ fx,
+                 float4* __restrict__ fy, const Consts c, int M, int N) {
+  __shared__ float4 P[11][35];
+  const int tx = threadIdx.x, ty = threadIdx.y, i0 = blockIdx.x * 32, j0 = blockIdx.y * 8;
+  const int i = i0 + tx, j = j0 + ty;
+  const bool jf = i < M && j <= N, jn = i < M && j < N;
+  float nx = 0, ny = 0, mx = 0, my = 0, len;
+  if (jf) edge_normal<false>(V[(size_t)j * M + i], V[(size_t)j * M + (i + 1) % M], nx, ny, len);
+  if (jn) edge_normal<false>(V[(size_t)(j + 1) * M + i], V[(size_t)j * M + i], mx, my, len);
+  grid_dep_wait();
+  grid_dep_launch();
+  for (int k = ty * 32 + tx; k < 11 * 35; k += 256) {
+    const int r = k / 35, cc = k % 35;
+    if (j0 - 2 + r <= N + 1 && i0 - 2 + cc <= M)
+      P[r][cc] = to_prim<false>(ref_load(st, V, c, M, N, i0 - 2 + cc, j0 - 2 + r), c.gm1);
+  }
+  __syncthreads();
+  if (jf)
+    fy[(size_t)j * M + i] = face_flux<SCHEME>(P[ty][tx + 2], P[ty + 1][tx + 2], P[ty + 2][tx + 2], P[ty + 3][tx + 2], nx, ny, c);
+  if (jn)
+    fx[(size_t)j * M + i] = face_flux<SCHEME>(P[ty + 2][tx], P[ty + 2][tx + 1], P[ty + 2][tx + 2], P[ty + 2][tx + 3], mx, my, c);
 }
 
-template <int SCHEME>
-__global__ void k_ref_flux_i(const float4* __restrict__ st, const float2* __restrict__ V, float4* __restrict__ fx,
-                             const Consts c, int M, int N) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= M || j >= N) return;
-  float nx, ny, len;
-  edge_normal<false>(V[(size_t)(j + 1) * M + i], V[(size_t)j * M + i], nx, ny, len);
-  const float gm1 = c.gm1;
-  float4 f = face_flux<SCHEME>(to_prim<false>(ref_load(st, M, i - 2, j), gm1),
-                                      to_prim<false>(ref_load(st, M, i - 1, j), gm1),
-                                      to_prim<false>(ref_load(st, M, i, j), gm1),
-                                      to_prim<false>(ref_load(st, M, i + 1, j), gm1), nx, ny, c);
-  fx[(size_t)j * M + i] = f;
-}
-
-__global__ void k_ref_residual(const float4* __restrict__ fx, const float4* __restrict__ fy,
-                               const float4* __restrict__ flen, const float* __restrict__ area,
-                               float4* __restrict__ res, int M, int N) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
-  if (i >= M || j >= N) return;
+// residual of a cell from its faces (ausm.js:402-436)
+__device__ __forceinline__ float4 residual_of(const float4* __restrict__ fx, const float4* __restrict__ fy,
+                                              const float4* __restrict__ flen, const float* __restrict__ area, int M,
+                                              int i, int j) {
   size_t k = (size_t)j * M + i;
   float4 xl = fx[k], xr = fx[(size_t)j * M + (i + 1) % M], yu = fy[(size_t)(j + 1) * M + i], yd = fy[k];
   float4 l = flen[k];
@@ -99,33 +111,51 @@ __global__ void k_ref_residual(const float4* __restrict__ fx, const float4* __re
   R.y = -(xr.y * l.y - xl.y * l.x + yu.y * l.z - yd.y * l.w) / A;
   R.z = -(xr.z * l.y - xl.z * l.x + yu.z * l.z - yd.z * l.w) / A;
   R.w = -(xr.w * l.y - xl.w * l.x + yu.w * l.z - yd.w * l.w) / A;
-  res[k] = R;
+  return R;
 }
-
-template <int STAGE>
-__global__ void k_ref_rk(const float4* __restrict__ res, const float4* __restrict__ s0, const float4* __restrict__ s1,
-                         float4* __restrict__ out, const float* __restrict__ dtp, int M, int N) {
+__global__ void k_ref_residual(const float4* __restrict__ fx, const float4* __restrict__ fy,
+                               const float4* __restrict__ flen, const float* __restrict__ area,
+                               float4* __restrict__ res, int M, int N) {
   int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
   if (i >= M || j >= N) return;
+  grid_dep_wait();
+  grid_dep_launch();
+  res[(size_t)j * M + i] = residual_of(fx, fy, flen, area, M, i, j);
+}
+
+// residual and RK stage (ausm.js:402-527) of the interior rows; the residual, which only
+// this stage uses, stays in registers
+template <int STAGE>
+__global__ void k_ref_stage(const float4* __restrict__ fx, const float4* __restrict__ fy,
+                            const float4* __restrict__ flen, const float* __restrict__ area, const float4* s0,
+                            const float4* __restrict__ s1, float4* out, const float* __restrict__ dtp, int M,
+                            int N) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+  if (i >= M || j >= N) return;
+  grid_dep_wait();
+  grid_dep_launch();
   const float dt = *dtp;
-  size_t k = (size_t)j * M + i, o = (size_t)(j + 1) * M + i;
-  float4 R = res[k], Q = s0[o], o4;
+  size_t o = (size_t)(j + 1) * M + i;
+  const float4 Rr = residual_of(fx, fy, flen, area, M, i, j), Q = s0[o];
+  float4 o4;
   if constexpr (STAGE == 1) {
-    o4 = make_float4(Q.x + dt * R.x, Q.y + dt * R.y, Q.z + dt * R.z, Q.w + dt * R.w);
+    o4 = make_float4(Q.x + dt * Rr.x, Q.y + dt * Rr.y, Q.z + dt * Rr.z, Q.w + dt * Rr.w);
   } else if constexpr (STAGE == 2) {
     float4 Q1 = s1[o];
-    o4 = make_float4(0.75f * Q.x + 0.25f * (Q1.x + dt * R.x), 0.75f * Q.y + 0.25f * (Q1.y + dt * R.y),
-                     0.75f * Q.z + 0.25f * (Q1.z + dt * R.z), 0.75f * Q.w + 0.25f * (Q1.w + dt * R.w));
+    o4 = make_float4(0.75f * Q.x + 0.25f * (Q1.x + dt * Rr.x), 0.75f * Q.y + 0.25f * (Q1.y + dt * Rr.y),
+                     0.75f * Q.z + 0.25f * (Q1.z + dt * Rr.z), 0.75f * Q.w + 0.25f * (Q1.w + dt * Rr.w));
   } else {
     float4 Q2 = s1[o];
-    o4 = make_float4((Q.x + 2.0f * (Q2.x + dt * R.x)) / 3.0f, (Q.y + 2.0f * (Q2.y + dt * R.y)) / 3.0f,
-                     (Q.z + 2.0f * (Q2.z + dt * R.z)) / 3.0f, (Q.w + 2.0f * (Q2.w + dt * R.w)) / 3.0f);
+    o4 = make_float4((Q.x + 2.0f * (Q2.x + dt * Rr.x)) / 3.0f, (Q.y + 2.0f * (Q2.y + dt * Rr.y)) / 3.0f,
+                     (Q.z + 2.0f * (Q2.z + dt * Rr.z)) / 3.0f, (Q.w + 2.0f * (Q2.w + dt * Rr.w)) / 3.0f);
   }
   out[o] = o4;
 }
 
 __global__ void k_ref_wave(const float4* __restrict__ st, const float4* __restrict__ flen,
                            const float* __restrict__ area, float gamma, int M, int N, uint32_t* wave) {
+  grid_dep_wait();
+  grid_dep_launch();
   uint32_t wm = 0u;
   size_t total = (size_t)M * N;
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < total; k += (size_t)gridDim.x * blockDim.x) {
@@ -150,39 +180,28 @@ void launch_ref_metrics(const float2* V, float* area, float4* flen, int M, int N
 }
 void launch_ref_boundary(const float4* in, float4* out, const float2* V, const Consts& c, int M, int N,
                          cudaStream_t s) {
-  k_ref_boundary<<<grid16(M, N + 3), B16, 0, s>>>(in, out, V, c, M, N);
+  launch_pdl(k_ref_boundary, grid16(M, N + 3), B16, 0, s, in, out, V, c, M, N);
 }
 void launch_ref_fluxes(int scheme, const float4* st, const float2* V, float4* fx, float4* fy, const Consts& c, int M,
                        int N, cudaStream_t s) {
-  switch (scheme) {
-    case 0:
-      k_ref_flux_j<0><<<grid16(M, N + 1), B16, 0, s>>>(st, V, fy, c, M, N);
-      k_ref_flux_i<0><<<grid16(M, N), B16, 0, s>>>(st, V, fx, c, M, N);
-      break;
-    case 1:
-      k_ref_flux_j<1><<<grid16(M, N + 1), B16, 0, s>>>(st, V, fy, c, M, N);
-      k_ref_flux_i<1><<<grid16(M, N), B16, 0, s>>>(st, V, fx, c, M, N);
-      break;
-    default:
-      k_ref_flux_j<2><<<grid16(M, N + 1), B16, 0, s>>>(st, V, fy, c, M, N);
-      k_ref_flux_i<2><<<grid16(M, N), B16, 0, s>>>(st, V, fx, c, M, N);
-      break;
-  }
+  const dim3 g((M + 31) / 32, (N + 8) / 8), b(32, 8);
+  if (scheme == 0) launch_pdl(k_ref_fluxes<0>, g, b, 0, s, st, V, fx, fy, c, M, N);
+  else if (scheme == 1) launch_pdl(k_ref_fluxes<1>, g, b, 0, s, st, V, fx, fy, c, M, N);
+  else launch_pdl(k_ref_fluxes<2>, g, b, 0, s, st, V, fx, fy, c, M, N);
 }
 void launch_ref_residual(const float4* fx, const float4* fy, const float4* flen, const float* area, float4* res, int M,
                          int N, cudaStream_t s) {
-  k_ref_residual<<<grid16(M, N), B16, 0, s>>>(fx, fy, flen, area, res, M, N);
+  launch_pdl(k_ref_residual, grid16(M, N), B16, 0, s, fx, fy, flen, area, res, M, N);
 }
-void launch_ref_rk(int stage, const float4* res, const float4* s0, const float4* s1, float4* out, const float* dt,
-                   int M, int N, cudaStream_t s) {
-  if (stage == 1) k_ref_rk<1><<<grid16(M, N), B16, 0, s>>>(res, s0, s1, out, dt, M, N);
-  else if (stage == 2) k_ref_rk<2><<<grid16(M, N), B16, 0, s>>>(res, s0, s1, out, dt, M, N);
-  else k_ref_rk<3><<<grid16(M, N), B16, 0, s>>>(res, s0, s1, out, dt, M, N);
+void launch_ref_stage(int stage, const float4* fx, const float4* fy, const float4* flen, const float* area,
+                      const float4* s0, const float4* s1, float4* out, const float* dt, int M, int N, cudaStream_t s) {
+  auto k = stage == 1 ? k_ref_stage<1> : (stage == 2 ? k_ref_stage<2> : k_ref_stage<3>);
+  launch_pdl(k, grid16(M, N), B16, 0, s, fx, fy, flen, area, s0, s1, out, dt, M, N);
 }
 void launch_ref_wave(const float4* st, const float4* flen, const float* area, float gamma, int M, int N,
                      uint32_t* wave, cudaStream_t s) {
   int blocks = (int)std::min<size_t>(((size_t)M * N + 255) / 256, 148 * 8);
-  k_ref_wave<<<blocks, 256, 0, s>>>(st, flen, area, gamma, M, N, wave);
+  launch_pdl(k_ref_wave, dim3(blocks), dim3(256), 0, s, st, flen, area, gamma, M, N, wave);
 }
 void launch_dt(const uint32_t* wave, float* dt, float maxdt, float cfl, cudaStream_t s) {
   k_dt<<<1, 1, 0, s>>>(wave, dt, maxdt, cfl);
