@@ -115,7 +115,8 @@ __device__ __forceinline__ FaceW own_weights(const float4 (*Ti)[TX + 1], const f
 
 // Flux x length of every face of the tile, written over the face's record.  Face rows
 // ty and ty + TY/2 of each direction per thread; warp 1 also takes the right face
-// column (rows 0..TY-1), warp 0 the top face row.  INNER: the tile with its halo lies
+// column (rows 0..TY-1), the last warp the top face row: warp 0, whose first thread issues
+// the tile's copies and waits for them, has no extra work.  INNER: the tile with its halo lies
 // inside the grid away from the seam, so every face exists and no bound is tested.
 template <int SCHEME, int TY, bool INNER = false>
 __device__ __forceinline__ void faces_phase(const float4 (*P)[TX + 4], float4 (*Ti)[TX + 1], float4 (*Tj)[TX],
@@ -140,7 +141,7 @@ __device__ __forceinline__ void faces_phase(const float4 (*P)[TX + 4], float4 (*
   if (ty == 1 && tx < TY) iface(tx, TX);
 #pragma unroll
   for (int t = 0; t < 2; t++) jface(ty + NWY * t, tx);
-  if (ty == 0) jface(TY, tx);
+  if (ty == NWY - 1) jface(TY, tx);
 }
 
 // x / 3 correctly rounded (in all but rare halfway cases), as the reference's division:
