@@ -398,7 +398,7 @@ int ausm_destroy(ausm_solver* h) {
   if (h->counted) resident_user(h->dev, -1);
   if (h->st) cudaStreamSynchronize(h->st);
   void* dptrs[] = {h->V, h->Vd, h->Mi, h->Mj, h->Q[0], h->Q[1], h->Q[2], h->S[0], h->S[1], h->S[2], h->fx, h->fy, h->res,
-                   h->flen, h->area, h->staging, h->cp, h->wave, h->dt, h->dacc, h->parts, h->move, h->err_flag};
+                   h->flen, h->area, h->staging, h->cp, h->wave, h->dt, h->parts, h->move, h->err_flag};
   for (void* d : dptrs)
     if (d) cudaFree(d);
   delete h->f64;
@@ -451,7 +451,6 @@ int ausm_create(int M, int N, ausm_solver** out) {
   for (auto& q : h->Q) TRY(dalloc(&q, n));
   TRY(dalloc(&h->wave, 4));
   TRY(dalloc(&h->dt, 4));
-  TRY(dalloc(&h->dacc, 4));
   TRY(dalloc(&h->parts, 2 * (size_t)kMaxParts));
   TRY(dalloc(&h->move, 4));
   TRY(dalloc(&h->err_flag, 1));
@@ -950,12 +949,11 @@ int ausm_forces(ausm_solver* h, double* out6, double* cp) {
   double q_inf = 0.5 * p.in_rho * (vx * vx + vy * vy);
   if (cp && !h->cp) CU(h, dalloc(&h->cp, (size_t)h->M));
   if (h->engine == AUSM_ENGINE_F64)
-    h->f64->forces(h->Vd, h->parts, h->dacc, cp ? h->cp : nullptr, q_inf, p.in_pressure, h->st);
+    h->f64->forces(h->Vd, h->parts, h->wave + 3, h->h_acc, cp ? h->cp : nullptr, q_inf, p.in_pressure, h->st);
   else
-    launch_forces(interior(h), h->Vd, h->c, h->M, h->dacc, h->parts, cp ? h->cp : nullptr, q_inf, p.in_pressure,
-                  h->st);
+    launch_forces(interior(h), h->Vd, h->c, h->M, h->h_acc, h->parts, h->wave + 3, cp ? h->cp : nullptr, q_inf,
+                  p.in_pressure, h->st);
   CHECK_LAUNCH(h);
-  CU(h, cudaMemcpyAsync(h->h_acc, h->dacc, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->st));
   if (cp) CU(h, cudaMemcpyAsync(cp, h->cp, (size_t)h->M * sizeof(double), cudaMemcpyDeviceToHost, h->st));
   if ((rc = sync_and_check(h))) return rc;
   double Fx = h->h_acc[0], Fy = h->h_acc[1];
@@ -985,7 +983,7 @@ int ausm_residual_l2(ausm_solver* h, double* l2) {
   const float4* R = nullptr;
   if (h->engine == AUSM_ENGINE_F64) {
     h->f64->residual(h->p.scheme, h->Vd, h->st);
-    h->f64->sumsq_rho(h->parts, h->dacc, h->st);
+    h->f64->sumsq_rho(h->parts, h->wave + 3, h->h_acc, h->st);
   } else if (h->engine == AUSM_ENGINE_FUSED) {
     float4* scratch = h->Q[(h->cur + 1) % 3];
     launch_fused_stage(h->p.scheme, 0, false, h->Q[h->cur], nullptr, scratch, h->Mi, h->Mj, h->dt, h->wave, 0, h->c, M,
@@ -996,9 +994,8 @@ int ausm_residual_l2(ausm_solver* h, double* l2) {
     launch_ref_residual(h->fx, h->fy, h->flen, h->area, h->res, M, N, h->st);
     R = h->res;
   }
-  if (R) launch_sumsq_rho(R, (size_t)M * N, h->dacc, h->parts, h->st);
+  if (R) launch_sumsq_rho(R, (size_t)M * N, h->h_acc, h->parts, h->wave + 3, h->st);
   CHECK_LAUNCH(h);
-  CU(h, cudaMemcpyAsync(h->h_acc, h->dacc, sizeof(double), cudaMemcpyDeviceToHost, h->st));
   if ((rc = sync_and_check(h))) return rc;
   *l2 = std::sqrt(h->h_acc[0] / ((double)M * N));
   if (!std::isfinite(*l2)) return fail(h, AUSM_ERR_DIVERGED, "residual norm is not finite: the solution diverged");

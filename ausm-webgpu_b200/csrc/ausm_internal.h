@@ -58,7 +58,7 @@ __device__ __forceinline__ void block_max_to(uint32_t* dst, uint32_t v) {
 }
 
 // Block-wide sum of doubles, stored by one thread into *dst (a per-block slot; the
-// slots are then summed in a fixed order by launch_sum_parts, so the total does not
+// slots are then summed in a fixed order by sum_parts_last, so the total does not
 // depend on block timing).  All threads call it.
 __device__ __forceinline__ void block_sum_store(double* dst, double v) {
   __shared__ double warp_sum[32];
@@ -76,6 +76,36 @@ __device__ __forceinline__ void block_sum_store(double* dst, double v) {
 }
 // Per-block partial sums of a reduction (at most kMaxParts blocks per quantity).
 constexpr int kMaxParts = 148 * 16;
+// The last of the launch's nb blocks (256 threads each) to get here sums the slots:
+// out[q] = parts[q * kMaxParts + 0 .. nb - 1] in a fixed order (strided partial sums, then a
+// shared-memory tree), q < nq; out is pinned host memory, so no copy follows.  *ticket is
+// zero before and after.  (A second kernel for the sums and a copy of them took a call for
+// the forces 6 us more.)  All threads call it.
+__device__ __forceinline__ void sum_parts_last(const double* parts, int nb, int nq, uint32_t* ticket, double* out) {
+  __shared__ double sh[256];
+  __shared__ bool last;
+  const int t = threadIdx.x;
+  if (t == 0) {  // which stored this block's slots
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == (uint32_t)nb - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int q = 0; q < nq; q++) {
+    double a = 0.0;
+    for (int k = t; k < nb; k += 256) a += __ldcg(&parts[(size_t)q * kMaxParts + k]);
+    sh[t] = a;
+    __syncthreads();
+    for (int w = 128; w > 0; w >>= 1) {
+      if (t < w) sh[t] += sh[t + w];
+      __syncthreads();
+    }
+    if (t == 0) out[q] = sh[0];
+    __syncthreads();
+  }
+  if (t == 0) *ticket = 0u;
+}
 
 // ---- fused engine (kernels_fused.cu) ----
 // TMA descriptors of one solve for one tile height ty: per state buffer the halo box
@@ -213,11 +243,10 @@ struct F64Engine {
   void wave_speed(cudaStream_t s);
   void step(int scheme, int n, const double2* Vd, cudaStream_t s);
   void residual(int scheme, const double2* Vd, cudaStream_t s);  // dQ/dt of S[2] into res
-  void sumsq_rho(double* parts, double* acc, cudaStream_t s);
-  void forces(const double2* Vd, double* parts, double* acc, double* cp, double q_inf, double p_inf, cudaStream_t s);
+  void sumsq_rho(double* parts, uint32_t* ticket, double* acc, cudaStream_t s);
+  void forces(const double2* Vd, double* parts, uint32_t* ticket, double* acc, double* cp, double q_inf, double p_inf,
+              cudaStream_t s);
 };
-// out[q] = fixed-order sum of parts[q * kMaxParts + 0 .. nb - 1], q < nq (kernels_misc.cu)
-void launch_sum_parts(const double* parts, int nb, int nq, double* out, cudaStream_t s);
 
 // ---- reference-shaped engine (kernels_reference.cu, built with -fmad=false) ----
 // States use the reference layout [N+3][M] (row 0 wall ghost).
@@ -252,14 +281,15 @@ void launch_to_ref_layout(const float4* Qint, float4* ref, const float2* V, cons
                           cudaStream_t s);
 void launch_from_ref_layout(const float4* ref, float4* Qint, int M, int N, cudaStream_t s);
 void launch_fill(float4* Q, float4 v, size_t n, cudaStream_t s);
-// parts: 2 * kMaxParts doubles of scratch; acc gets the sums, in a fixed order.
 // FP64 face records: see k_metrics_d for their layout.
 void launch_d2f(const double2* a, float2* b, size_t n, cudaStream_t s);
 void launch_f2d(const float2* a, double2* b, size_t n, cudaStream_t s);
 void launch_metrics_d(const double2* V, float4* Mi, float4* Mj, int M, int N, cudaStream_t s);
+// parts: 2 * kMaxParts doubles of scratch; acc (pinned host memory) gets the sums, in a fixed
+// order (sum_parts_last).
 void launch_forces(const float4* row0, const double2* V, const Consts& c, int M, double* acc /*2*/, double* parts,
-                   double* cp, double q_inf, double p_inf, cudaStream_t s);
-void launch_sumsq_rho(const float4* R, size_t n, double* acc, double* parts, cudaStream_t s);
+                   uint32_t* ticket, double* cp, double q_inf, double p_inf, cudaStream_t s);
+void launch_sumsq_rho(const float4* R, size_t n, double* acc, double* parts, uint32_t* ticket, cudaStream_t s);
 void launch_field(const float4* Qint, const float2* V, const Consts& c, int kind, int M, int N, float* out,
                   cudaStream_t s);
 

@@ -196,7 +196,7 @@ __global__ void k_ex_from_f32(const float4* __restrict__ a, V4<R>* __restrict__ 
 // surface force from the FP64 state (pressure of interior row 1, graphs.js:5-41),
 // per-block partial sums; Cp per wall face
 __global__ void k_ex_forces(const V4<R>* __restrict__ row1, const V2<R>* __restrict__ V, R gamma, int M,
-                            double* parts, double* cp, double q_inf, double p_inf) {
+                            double* parts, double* cp, double q_inf, double p_inf, uint32_t* ticket, double* out) {
   double fx = 0.0, fy = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x) {
     V4<R> s = row1[i];
@@ -213,13 +213,15 @@ __global__ void k_ex_forces(const V4<R>* __restrict__ row1, const V2<R>* __restr
   block_sum_store(parts + blockIdx.x, fx);
   __syncthreads();
   block_sum_store(parts + kMaxParts + blockIdx.x, fy);
+  sum_parts_last(parts, gridDim.x, 2, ticket, out);
 }
 
-__global__ void k_ex_sumsq_rho(const V4<R>* __restrict__ res, size_t n, double* parts) {
+__global__ void k_ex_sumsq_rho(const V4<R>* __restrict__ res, size_t n, double* parts, uint32_t* ticket, double* out) {
   double s = 0.0;
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
     s += res[k].x * res[k].x;
   block_sum_store(parts + blockIdx.x, s);
+  sum_parts_last(parts, gridDim.x, 1, ticket, out);
 }
 
 inline dim3 grid16(int w, int h) { return dim3((w + 15) / 16, (h + 15) / 16); }
@@ -309,18 +311,16 @@ void F64Engine::residual(int scheme, const double2* Vd_, cudaStream_t s) {
   else fluxes<2>(S[2], Vd, fx, fy, c, M, N, s);
   launch_pdl(k_ex_residual, grid16(M, N), B16, 0, s, fx, fy, flen, area, res, M, N);
 }
-void F64Engine::sumsq_rho(double* parts, double* acc, cudaStream_t s) {
+void F64Engine::sumsq_rho(double* parts, uint32_t* ticket, double* acc, cudaStream_t s) {
   const size_t n = (size_t)M * N;
   const int blocks = grid1d(n);
-  k_ex_sumsq_rho<<<blocks, 256, 0, s>>>(res, n, parts);
-  launch_sum_parts(parts, blocks, 1, acc, s);
+  k_ex_sumsq_rho<<<blocks, 256, 0, s>>>(res, n, parts, ticket, acc);
 }
-void F64Engine::forces(const double2* Vd, double* parts, double* acc, double* cp, double q_inf, double p_inf,
+void F64Engine::forces(const double2* Vd, double* parts, uint32_t* ticket, double* acc, double* cp, double q_inf, double p_inf,
                        cudaStream_t s) {
   int blocks = std::min((M + 255) / 256, 148);
   k_ex_forces<<<blocks, 256, 0, s>>>(S[2] + M, reinterpret_cast<const V2<R>*>(Vd), c.gamma, M, parts, cp, q_inf,
-                                     p_inf);
-  launch_sum_parts(parts, blocks, 2, acc, s);
+                                     p_inf, ticket, acc);
 }
 
 }  // namespace ausm

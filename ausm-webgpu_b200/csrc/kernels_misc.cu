@@ -71,7 +71,7 @@ __global__ void k_metrics_d(const double2* __restrict__ V, float4* __restrict__ 
 // ---- surface force (graphs.js:5-41, summed as graphs.js:43-103): FP32 pressure of the first interior cell,
 // FP64 face length, normal and sum; also Cp per wall face ----
 __global__ void k_forces(const float4* __restrict__ row0, const double2* __restrict__ V, const Consts c, int M,
-                         double* parts, double* cp, double q_inf, double p_inf) {
+                         double* parts, double* cp, double q_inf, double p_inf, uint32_t* ticket, double* out) {
   double fx = 0.0, fy = 0.0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x) {
     float4 s = row0[i];
@@ -88,32 +88,17 @@ __global__ void k_forces(const float4* __restrict__ row0, const double2* __restr
   block_sum_store(parts + blockIdx.x, fx);
   __syncthreads();
   block_sum_store(parts + kMaxParts + blockIdx.x, fy);
+  sum_parts_last(parts, gridDim.x, 2, ticket, out);
 }
 
-__global__ void k_sumsq_rho(const float4* __restrict__ R, size_t n, double* parts) {
+__global__ void k_sumsq_rho(const float4* __restrict__ R, size_t n, double* parts, uint32_t* ticket, double* out) {
   double s = 0.0;
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
     double r = R[k].x;
     s += r * r;
   }
   block_sum_store(parts + blockIdx.x, s);
-}
-
-// out[q] = sum of parts[q * kMaxParts + 0 .. nb - 1], in a fixed order (one block of
-// 256 threads per quantity q: strided partial sums, then a shared-memory tree).
-__global__ void k_sum_parts(const double* __restrict__ parts, int nb, double* __restrict__ out) {
-  __shared__ double sh[256];
-  const int t = threadIdx.x;
-  const double* p = parts + (size_t)blockIdx.x * kMaxParts;
-  double a = 0.0;
-  for (int k = t; k < nb; k += 256) a += p[k];
-  sh[t] = a;
-  __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if (t < w) sh[t] += sh[t + w];
-    __syncthreads();
-  }
-  if (t == 0) out[blockIdx.x] = sh[0];
+  sum_parts_last(parts, gridDim.x, 1, ticket, out);
 }
 
 // ---- headless field output (ausm.js:617-707 without the colour map) ----
@@ -163,23 +148,18 @@ void launch_from_ref_layout(const float4* ref, float4* Qint, int M, int N, cudaS
 }
 void launch_fill(float4* Q, float4 v, size_t n, cudaStream_t s) { k_fill<<<grid1d(n), 256, 0, s>>>(Q, v, n); }
 void launch_forces(const float4* row0, const double2* V, const Consts& c, int M, double* acc, double* parts,
-                   double* cp, double q_inf, double p_inf, cudaStream_t s) {
+                   uint32_t* ticket, double* cp, double q_inf, double p_inf, cudaStream_t s) {
   int blocks = std::min((M + 255) / 256, 148);
-  k_forces<<<blocks, 256, 0, s>>>(row0, V, c, M, parts, cp, q_inf, p_inf);
-  k_sum_parts<<<2, 256, 0, s>>>(parts, blocks, acc);
+  k_forces<<<blocks, 256, 0, s>>>(row0, V, c, M, parts, cp, q_inf, p_inf, ticket, acc);
 }
-void launch_sumsq_rho(const float4* R, size_t n, double* acc, double* parts, cudaStream_t s) {
+void launch_sumsq_rho(const float4* R, size_t n, double* acc, double* parts, uint32_t* ticket, cudaStream_t s) {
   const int blocks = grid1d(n);  // <= kMaxParts
-  k_sumsq_rho<<<blocks, 256, 0, s>>>(R, n, parts);
-  k_sum_parts<<<1, 256, 0, s>>>(parts, blocks, acc);
+  k_sumsq_rho<<<blocks, 256, 0, s>>>(R, n, parts, ticket, acc);
 }
 void launch_d2f(const double2* a, float2* b, size_t n, cudaStream_t s) { k_d2f<<<grid1d(n), 256, 0, s>>>(a, b, n); }
 void launch_f2d(const float2* a, double2* b, size_t n, cudaStream_t s) { k_f2d<<<grid1d(n), 256, 0, s>>>(a, b, n); }
 void launch_metrics_d(const double2* V, float4* Mi, float4* Mj, int M, int N, cudaStream_t s) {
   k_metrics_d<<<grid16(M, N + 1), B16, 0, s>>>(V, Mi, Mj, M, N);
-}
-void launch_sum_parts(const double* parts, int nb, int nq, double* out, cudaStream_t s) {
-  k_sum_parts<<<nq, 256, 0, s>>>(parts, nb, out);
 }
 void launch_field(const float4* Qint, const float2* V, const Consts& c, int kind, int M, int N, float* out,
                   cudaStream_t s) {

@@ -32,9 +32,9 @@ struct ausm_solver {
   float* area = nullptr;
   float4* staging = nullptr;
   double* cp = nullptr;
-  uint32_t* wave = nullptr;    // [0] max wave speed bits; [1..2] the resident kernel's (kernels_resident.cu)
+  uint32_t* wave = nullptr;    // [0] max wave speed bits; [1..2] the resident kernel's (kernels_resident.cu); [3] the
+                               // finished blocks of a reduction (sum_parts_last)
   float* dt = nullptr;
-  double* dacc = nullptr;
   double* parts = nullptr;  // 2 * kMaxParts per-block partial sums
   uint32_t* move = nullptr;
   int* err_flag = nullptr;  // set by a kernel whose bounded wait gave up
@@ -44,7 +44,7 @@ struct ausm_solver {
   int tile_rows = 0;      // tile height of the TMA stage kernel; 0 until tuned
   float* h_dt = nullptr;
   uint32_t* h_wave = nullptr;
-  double* h_acc = nullptr;
+  double* h_acc = nullptr;  // pinned; sums of forces and norms, written by the kernels
   std::string err;
 };
 
