@@ -286,9 +286,9 @@ void launch_grid_init_d(double2* V, int M, int N, double first_spacing, cudaStre
   k_grid_guess<double2, double><<<dim3((M + 31) / 32, (N + kInitRows - 1) / kInitRows), 256, 0, s>>>(V, M, N, first_spacing);
 }
 
-// 8 sweeps (a halo of 8) in tiles of 48 x up to 48: us per sweep, one launch each / now:
-// 128 x 96 4.1 / 0.8, 512 x 384 4.1 / 1.8, 1024 x 768 8.2 / 4.8 (tiles of 32 rows 5.3).
-constexpr int kJacobiSweeps = 8;
+// 6 sweeps (a halo of 6) in tiles of 52 x up to 48: us per sweep, one launch each / now:
+// 128 x 96 4.1 / 0.8, 512 x 384 4.1 / 1.8, 1024 x 768 8.2 / 4.4 (8 sweeps 4.8).
+constexpr int kJacobiSweeps = 6;
 int grid_jacobi_sweeps() { return kJacobiSweeps; }
 void launch_grid_jacobi(const float2* src, float2* dst, const float2* ends, int M, int N, int sweeps, cudaStream_t s) {
   constexpr int NW = 16;
