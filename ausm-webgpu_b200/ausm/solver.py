@@ -144,8 +144,10 @@ class Solver:
         a = np.ascontiguousarray(xy, dtype=np.float32).reshape(self.N + 1, self.M, 2)
         self._c(lib().ausm_set_vertices(self.h, _fp(a)))
 
+    # Arrays the library fills whole are made uncleared: zeroing a new array and taking its
+    # page faults cost more than the copy (6.3 MB of vertices: 0.88 -> 0.36 ms).
     def vertices(self) -> np.ndarray:
-        a = np.zeros((self.N + 1, self.M, 2), dtype=np.float32)
+        a = np.empty((self.N + 1, self.M, 2), dtype=np.float32)
         self._c(lib().ausm_get_vertices(self.h, _fp(a)))
         return a
 
@@ -160,7 +162,7 @@ class Solver:
     def state(self, out: np.ndarray | None = None) -> np.ndarray:
         """State in the reference layout; `out` (float32, contiguous, e.g. pinned) is
         filled in place when given."""
-        a = np.zeros((self.N + 3, self.M, 4), dtype=np.float32) if out is None else out
+        a = np.empty((self.N + 3, self.M, 4), dtype=np.float32) if out is None else out
         if a.dtype != np.float32 or not a.flags.c_contiguous or a.size != (self.N + 3) * self.M * 4:
             raise AusmError(_lib.ERR_INVALID, "out must be a contiguous float32 array of (N+3)*M*4 values")
         self._c(lib().ausm_get_state(self.h, _fp(a)))
@@ -168,7 +170,7 @@ class Solver:
 
     def state_f64(self) -> np.ndarray:
         """State in the reference layout in double (the F64 engine's own; FP32 engines' widened)."""
-        a = np.zeros((self.N + 3, self.M, 4), dtype=np.float64)
+        a = np.empty((self.N + 3, self.M, 4), dtype=np.float64)
         self._c(lib().ausm_get_state_f64(self.h, _dp(a)))
         return a
 
@@ -206,7 +208,7 @@ class Solver:
         return r.value
 
     def field(self, kind: str = "density") -> np.ndarray:
-        a = np.zeros((self.N, self.M), dtype=np.float32)
+        a = np.empty((self.N, self.M), dtype=np.float32)
         self._c(lib().ausm_field(self.h, _lib.FIELDS[kind], _fp(a)))
         return a
 
