@@ -9,7 +9,7 @@
 // per colour or sweep.  One launch per colour left three lanes of four idle, read the
 // nine neighbours from L2 with a stride and cost a launch per colour.  Measured on B200,
 // FP64 multicolour, us per sweep before / now: 128 x 96 18.4 / 3.0, 512 x 384 25.1 / 5.5,
-// 1024 x 768 41.6 / 13.4, 4096 x 3072 563 / 184.  What is left at 1024 x 768: some 5 us of FP64
+// 1024 x 768 41.6 / 13.0, 4096 x 3072 563 / 168.  What is left at 1024 x 768: some 5 us of FP64
 // arithmetic (72 operations a vertex at half rate, halo and idle lanes included) and the
 // tiles' way in and out of L2, which all CTAs of the launch take at the same time; on
 // small grids the latency of the colour steps, 0.4 us each.
@@ -122,6 +122,32 @@ __device__ __forceinline__ const V2T* grid_row(const V2T* src, const V2T* ends, 
   return j == 0 ? ends : (j == N ? ends + (size_t)N * M : src + (size_t)(j - 1) * M);
 }
 
+// Fetches the tile's rows (with the halo) that the grid has, two columns gi[] per lane, and
+// hands them to put(tile row, grid row, values), eight loads of a lane in flight (against
+// row by row: multicolour 1024 x 768 13.4 -> 13.0, 4096 x 3072 184 -> 168 us per sweep).
+template <class V2T, int NW, class Put>
+__device__ __forceinline__ void load_rows(const GridTile& t, int H, const V2T* src, const V2T* ends, int M, int N,
+                                          const int (&gi)[2], int warp, Put put) {
+  constexpr int B = 4;
+  for (int r = warp; r < t.h + 2 * H; r += B * NW) {
+    V2T v[B][2];
+#pragma unroll
+    for (int q = 0; q < B; q++) {
+      const int j = t.j0 - H + r + q * NW;
+      if (r + q * NW < t.h + 2 * H && j >= 0 && j <= N) {
+        const V2T* row = grid_row(src, ends, M, N, j);
+        v[q][0] = row[gi[0]];
+        v[q][1] = row[gi[1]];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < B; q++) {
+      const int j = t.j0 - H + r + q * NW;
+      if (r + q * NW < t.h + 2 * H && j >= 0 && j <= N) put(r + q * NW, j, v[q]);
+    }
+  }
+}
+
 // FP64 multicolour Gauss-Seidel.  Colour (i & 1) * 2 + (j & 1); with odd M the seam column
 // i = M - 1 has the colours 4 + (j & 1), so no two vertices of a colour touch (9-point
 // stencil, periodic in i).  A row of the tile is one warp: lane k has the columns 2 k and
@@ -146,14 +172,10 @@ __global__ void __launch_bounds__(32 * NW)
   }
   grid_dep_wait();
   grid_dep_launch();
-  for (int r = warp; r < t.h + 2 * H; r += NW) {
-    const int j = t.j0 - H + r;
-    if (j >= 0 && j <= N) {
-      const double2* row = grid_row(src, ends, M, N, j);
+  load_rows<double2, NW>(t, H, src, ends, M, N, gi, warp, [&](int r, int, const double2* v) {
 #pragma unroll
-      for (int k = 0; k < 2; k++) at(r, 2 * lane + k) = row[gi[k]];
-    }
-  }
+    for (int k = 0; k < 2; k++) at(r, 2 * lane + k) = v[k];
+  });
   __syncthreads();
   const int steps = NC * sweeps;
   uint32_t mv = 0u;
@@ -204,18 +226,13 @@ __global__ void __launch_bounds__(32 * NW)
   }
   grid_dep_wait();
   grid_dep_launch();
-  for (int r = warp; r < rows; r += NW) {
-    const int j = t.j0 - H + r;
-    if (j >= 0 && j <= N) {
-      const float2* row = grid_row(src, ends, M, N, j);
+  load_rows<float2, NW>(t, H, src, ends, M, N, gi, warp, [&](int r, int j, const float2* v) {
 #pragma unroll
-      for (int k = 0; k < 2; k++) {
-        const float2 v = row[gi[k]];
-        a[r * GW + lane + 32 * k] = v;
-        if (j == 0 || j == N) b[r * GW + lane + 32 * k] = v;  // fixed rows, in both copies
-      }
+    for (int k = 0; k < 2; k++) {
+      a[r * GW + lane + 32 * k] = v[k];
+      if (j == 0 || j == N) b[r * GW + lane + 32 * k] = v[k];  // fixed rows, in both copies
     }
-  }
+  });
   __syncthreads();
   for (int st = 0; st < sweeps; st++) {
     const int e = sweeps - 1 - st;
@@ -272,7 +289,7 @@ void sweeps_d(const double2* src, double2* dst, const double2* ends, int M, int 
 // the SMs one each: there a launch is bound by its fixed cost and the latency of the colour
 // steps (us per sweep, one sweep / two: 128 x 96 3.6 / 3.0, 257 x 131 5.2 / 4.7, 512 x 384
 // 6.3 / 5.4; four: 3.5 and more).  Beyond, the wider tiles of one sweep (56 or 52 columns)
-// win: 1024 x 768 13.4 / 14.1.
+// win: 1024 x 768 13.4 / 14.1 (before the loads were batched).
 bool two_sweeps(int M, int N) {
   const int ti = GW - 2 * 2 * ((M & 1) ? 6 : 4);
   return (long long)((M + ti - 1) / ti) * ((N - 1 + 31) / 32) <= kSMs;
