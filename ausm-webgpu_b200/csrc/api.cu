@@ -819,13 +819,21 @@ int resident_height(ausm_solver* h, int* rows) {
   return AUSM_OK;
 }
 
-// n fused steps by the resident kernel.
-int resident_steps(ausm_solver* h, int n, int rows) {
+// n fused steps by the resident kernel.  *refused: the device would not take the launch (a
+// process that may use a part of the SMs only), nothing was done.
+int resident_steps(ausm_solver* h, int n, int rows, bool* refused) {
   for (int done = 0; done < n;) {
     const int k = std::min(n - done, kResidentSteps);
     const int to = (h->cur + k) % 3;
-    CU(h, launch_resident(h->p.scheme, h->Q[h->cur], h->Q[to], h->Mi, h->Mj, h->dt, h->wave, rows, k, done == 0,
-                          done + k == n, h->h_dt, (int*)h->h_wave + 2, h->err_flag, h->c, h->M, h->N, h->st));
+    const cudaError_t e =
+        launch_resident(h->p.scheme, h->Q[h->cur], h->Q[to], h->Mi, h->Mj, h->dt, h->wave, rows, k, done == 0,
+                        done + k == n, h->h_dt, (int*)h->h_wave + 2, h->err_flag, h->c, h->M, h->N, h->st);
+    if (done == 0 && e == cudaErrorCooperativeLaunchTooLarge) {
+      cudaGetLastError();
+      *refused = true;
+      return AUSM_OK;
+    }
+    CU(h, e);
     h->cur = to;
     done += k;
   }
@@ -858,8 +866,9 @@ int step_impl(ausm_solver* h, int n, float* dt_out, bool read_err) {
   }
   int res_rows = 0;
   if (h->engine == AUSM_ENGINE_FUSED && n > 0 && (rc = resident_height(h, &res_rows))) return rc;
-  if (res_rows) {
-    if ((rc = resident_steps(h, n, res_rows))) return rc;
+  bool refused = false;
+  if (res_rows && (rc = resident_steps(h, n, res_rows, &refused))) return rc;
+  if (res_rows && !refused) {
     ramp_after_steps(h, n);
     h->err_read_queued = true;
     return dt_out ? read_dt(h, dt_out) : AUSM_OK;

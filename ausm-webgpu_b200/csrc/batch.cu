@@ -413,13 +413,20 @@ int sync_and_check(ausm_batch* b) {
 }
 
 // n steps of every member by resident launches, then the rotation and the gather as in
-// enqueue_steps.
-int resident_steps(ausm_batch* b, int n) {
+// enqueue_steps.  *refused as in api.cu.
+int resident_steps(ausm_batch* b, int n, bool* refused) {
   const int ns = (int)b->members.size();
   for (int done = 0; done < n;) {
     const int k = std::min(n - done, ausm::kResidentSteps);
-    BCU(b, ausm::launch_resident_batch(b->d_solves, b->d_ritems, (int)b->ritems.size(), b->res_rows, ns, k, done == 0,
-                                       done + k == n, b->d_err, b->st));
+    const cudaError_t e =
+        ausm::launch_resident_batch(b->d_solves, b->d_ritems, (int)b->ritems.size(), b->res_rows, ns, k, done == 0,
+                                    done + k == n, b->d_err, b->st);
+    if (done == 0 && e == cudaErrorCooperativeLaunchTooLarge) {
+      cudaGetLastError();
+      *refused = true;
+      return AUSM_OK;
+    }
+    BCU(b, e);
     ausm::launch_batch_advance(b->d_solves, ns, k, b->d_steps, b->st);
     done += k;
   }
@@ -580,13 +587,14 @@ int batch_step_impl(ausm_batch* b, int n, float* dt_wave, bool read_err) {
   for (ausm_solver* h : b->members)
     BNEED(b, h->has_grid && h->has_state, AUSM_ERR_STATE, "a member lost its grid or state");
   // members whose tiles all fit on the chip together step in one launch
-  const bool fixed = ausm::forced_tile_rows() != 0;
-  if ((fixed || !b->res_rows) && (rc = tune_rows(b))) return rc;
-  rc = sync_descriptors(b);
-  if (rc) return rc;
-  const bool resident = !fixed && b->res_rows != 0;
-  rc = resident ? resident_steps(b, n) : run_steps(b, n);
-  if (rc) return rc;
+  bool resident = !ausm::forced_tile_rows() && b->res_rows != 0, refused = false;
+  if (resident) {
+    if ((rc = sync_descriptors(b)) || (rc = resident_steps(b, n, &refused))) return rc;
+    resident = !refused;
+  }
+  if (!resident) {
+    if ((rc = tune_rows(b)) || (rc = sync_descriptors(b)) || (rc = run_steps(b, n))) return rc;
+  }
   for (size_t k = 0; k < b->members.size(); k++) {
     ausm_solver* h = b->members[b->order[k]];
     h->cur = (h->cur + n) % 3;
