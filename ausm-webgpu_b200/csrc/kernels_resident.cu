@@ -246,19 +246,57 @@ __device__ __forceinline__ void resident_tile(Smem<TY>& sm, const Job& b, const 
   bool ok = true;
   int rk = 1;
   for (int st = 0; st < stages; st++) {
-    if (EARLY && ty < RW) {
-      __syncwarp();  // the own row of P
-      if (tx >= 2 && tx <= w - 2) iface(ty, tx);
-    }
-    if (fetch && (st > 0 || in_place)) {  // the neighbours' edges
-      const uint32_t tag = tag0 + st;
-      const ulonglong2* e = from + (tag & 1u) * (2 * E::NC);
-      const unsigned polls = c_wait_polls * 64u;
+    const bool wants = fetch && (st > 0 || in_place);  // the neighbours' edges
+    const uint32_t tag = tag0 + st;
+    const ulonglong2* e = from + (tag & 1u) * (2 * E::NC);
+    const unsigned polls = c_wait_polls * 64u;
+    auto arrived = [&](ulonglong2 x, ulonglong2 y) {
+      if (tag_of(x.x) != tag || tag_of(x.y) != tag || tag_of(y.x) != tag || tag_of(y.y) != tag) return false;
+      *halo = make_float4(value_of(x.x), value_of(x.y), value_of(y.x), value_of(y.y));
+      return true;
+    };
+    if constexpr (EARLY) {
+      // The edges are asked for in the middle of the early face: by the time the words are
+      // read in L2 they have mostly arrived, and the answer is back soon after the face is
+      // done (asked for after the face: 1.54 us a stage instead of 1.44).
+      ulonglong2 x{}, y{};
+      if (ty < RW) {
+        __syncwarp();  // the own row of P
+        const bool inner = tx >= 2 && tx <= w - 2;
+        float4 L, R;
+        if (inner) {
+          const float4* p = &sm.P[ty + 2][tx];
+          face_states<SF>(p[0], p[1], p[2], p[3], c, L, R);
+        }
+        if (wants) {
+          x = ld_pair(e);
+          y = ld_pair(e + E::NC);
+        }
+        if (inner) {
+          const float4 m = sm.Ti[ty][tx];
+          sm.Fi[ty][tx] = face_flux_states<SF>(L, R, m.x, m.y, m.z, c);
+        }
+      } else if (wants) {
+        x = ld_pair(e);
+        y = ld_pair(e + E::NC);
+      }
+      if (wants) {
+        ok = false;
+        for (unsigned it = 0; it < polls; it++) {
+          if (arrived(x, y)) {
+            ok = true;
+            break;
+          }
+          if ((it & 1023u) == 1023u && *(volatile int*)err) break;
+          x = ld_pair(e);
+          y = ld_pair(e + E::NC);
+        }
+      }
+    } else if (wants) {
       ok = false;
       for (unsigned it = 0; it < polls; it++) {
         const ulonglong2 x = ld_pair(e), y = ld_pair(e + E::NC);
-        if (tag_of(x.x) == tag && tag_of(x.y) == tag && tag_of(y.x) == tag && tag_of(y.y) == tag) {
-          *halo = make_float4(value_of(x.x), value_of(x.y), value_of(y.x), value_of(y.y));
+        if (arrived(x, y)) {
           ok = true;
           break;
         }

@@ -326,18 +326,8 @@ __device__ __forceinline__ float4 face_flux(float4 L2, float4 L, float4 R, float
 // SCHEME_FLAGS: the scheme (bits 0-1), plus 4 when the launch knows MUSCL is on, so the
 // kernel has no per-face branch on it (c.muscl is read at run time otherwise).
 template <int SCHEME_FLAGS>
-__device__ __forceinline__ float4 face_flux_len(float4 L2, float4 L, float4 R, float4 R2, float nx, float ny,
-                                                float hl, const Consts& c) {
+__device__ __forceinline__ float4 face_flux_states(float4 Lm, float4 Rm, float nx, float ny, float hl, const Consts& c) {
   constexpr int SCHEME = SCHEME_FLAGS & 3;
-  constexpr bool MUSCL_ON = (SCHEME_FLAGS & 4) != 0;  // MUSCL known on at compile time
-  float4 Lm = L, Rm = R;
-  if (MUSCL_ON || c.muscl > 0) {
-    float2 a, b;
-    muscl2_packed(lo2(L2), lo2(L), lo2(R), lo2(R2), a, b);
-    Lm.x = a.x; Lm.y = a.y; Rm.x = b.x; Rm.y = b.y;
-    muscl2_packed(hi2(L2), hi2(L), hi2(R), hi2(R2), a, b);
-    Lm.z = a.x; Lm.w = a.y; Rm.z = b.x; Rm.w = b.y;
-  }
   const float rhoL = Lm.x, rhoR = Rm.x, pL = Lm.w, pR = Rm.w;
   const float vxL = Lm.y, vyL = Lm.z, vxR = Rm.y, vyR = Rm.z;
   const float uL = fmaf(vyL, ny, vxL * nx), uR = fmaf(vyR, ny, vxR * nx);
@@ -413,6 +403,30 @@ __device__ __forceinline__ float4 face_flux_len(float4 L2, float4 L, float4 R, f
     const float p1 = left ? vxL : vxR, p2 = left ? vyL : vyR, p3 = left ? h2L : h2R;
     return make_float4(ml, fmaf(p1, ml, nx * Pl), fmaf(p2, ml, ny * Pl), p3 * (0.5f * ml));
   }
+}
+
+// ... of the face states of the four cells along the face normal line (MUSCL, or the two
+// cells themselves without it)
+template <int SCHEME_FLAGS>
+__device__ __forceinline__ void face_states(float4 L2, float4 L, float4 R, float4 R2, const Consts& c, float4& Lm,
+                                            float4& Rm) {
+  constexpr bool MUSCL_ON = (SCHEME_FLAGS & 4) != 0;  // MUSCL known on at compile time
+  Lm = L;
+  Rm = R;
+  if (MUSCL_ON || c.muscl > 0) {
+    float2 a, b;
+    muscl2_packed(lo2(L2), lo2(L), lo2(R), lo2(R2), a, b);
+    Lm.x = a.x; Lm.y = a.y; Rm.x = b.x; Rm.y = b.y;
+    muscl2_packed(hi2(L2), hi2(L), hi2(R), hi2(R2), a, b);
+    Lm.z = a.x; Lm.w = a.y; Rm.z = b.x; Rm.w = b.y;
+  }
+}
+template <int SCHEME_FLAGS>
+__device__ __forceinline__ float4 face_flux_len(float4 L2, float4 L, float4 R, float4 R2, float nx, float ny,
+                                                float hl, const Consts& c) {
+  float4 Lm, Rm;
+  face_states<SCHEME_FLAGS>(L2, L, R, R2, c, Lm, Rm);
+  return face_flux_states<SCHEME_FLAGS>(Lm, Rm, nx, ny, hl, c);
 }
 
 // Cell wave speed for the CFL condition (ausm.js:617-630): (|v| + a) * sum(l) / (2 A).
