@@ -37,13 +37,15 @@
 // interleaved, the fifth takes the top row and the right column; more work per warp and
 // no early faces (they were 5 % slower there: other CTAs of the SM fill the wait).
 //
-// Measured on B200 (us per stage; stage kernels before / 4 rows / 8 rows), SLAU2, MUSCL:
-//     64 x 33    4.55 / 1.44 / 2.33
-//    128 x 96    4.32 / 1.47 / 2.38
-//    257 x 131   4.59 / 1.70 / 2.53
-//    333 x 250   5.30 / 2.44 / 3.01
-//    512 x 384   8.02 /  --  / 4.58   (43 G cell-stages/s)
-// Bound by latency: of about 2800 cycles of a 4-row stage on an idle chip some 1600 pass
+// Measured on B200 (us per stage; stage kernels / this one), SLAU2, MUSCL:
+//     64 x 33    4.55 / 1.37 (4 rows)
+//    128 x 96    4.32 / 1.37
+//    257 x 131   4.59 / 1.61
+//    333 x 250   5.30 / 2.47
+//    460 x 340    --  / 3.94 (8 rows)
+//    512 x 384   8.02 / 4.63   (42 G cell-stages/s)
+// (8-row tiles where 4 rows fit: 128 x 96 2.4, 257 x 131 2.5, 333 x 250 2.9.)
+// Bound by latency: of about 2600 cycles of a 4-row stage on an idle chip some 1400 pass
 // between publishing an edge and having the neighbours' (two L2 trips, with the early
 // faces inside), 600 in one face evaluation and 600 in the combination.  At 512 x 384 the
 // fullest SM holds 6 tiles and issues about 60 % of the time.
@@ -65,7 +67,14 @@ constexpr int RW = 4;  // warps that own cells
 // ... and warps that fetch the halo and share the last faces: two where each owning warp
 // has one row, so that none of them has two faces in a row there
 constexpr int aux_warps(int TY) { return TY == 4 ? 2 : 1; }
-constexpr int kMaxTiles4 = 5 * 148, kMaxTiles8 = 6 * 148;  // tiles of a launch (an exchange buffer's size)
+// Each height is built twice: for one CTA per SM fewer than would fit, with registers to
+// interleave more of a face's arithmetic, and for all that fit.  A launch takes the first
+// while its tiles fit (us per stage, all that fit / fewer: 128 x 96 1.45 / 1.37, 257 x 131
+// 1.77 / 1.61, 300 x 220 2.14 / 2.04; 8 rows: 460 x 340 4.12 / 3.94, 400 x 380 AUSM+-up
+// 4.37 / 4.09; three CTAs of 4 rows instead of four gain another 1-2 % on the smallest).
+constexpr int few_ctas(int TY) { return TY == 4 ? 4 : 5; }
+constexpr int more_ctas(int TY) { return TY == 4 ? 5 : 6; }
+constexpr int kMaxTiles4 = more_ctas(4) * 148, kMaxTiles8 = more_ctas(8) * 148;  // tiles of a launch
 constexpr int threads_of(int TY) { return 32 * (RW + aux_warps(TY)); }
 
 // Exchange cells of one tile and parity: bottom rows 2 x 32, top rows 2 x 32, left
@@ -258,7 +267,7 @@ __device__ __forceinline__ void resident_tile(Smem<TY>& sm, const Job& b, const 
     if constexpr (EARLY) {
       // The edges are asked for in the middle of the early face: by the time the words are
       // read in L2 they have mostly arrived, and the answer is back soon after the face is
-      // done (asked for after the face: 1.54 us a stage instead of 1.44).
+      // done (asked for after the face: 7 % more a stage).
       ulonglong2 x{}, y{};
       if (ty < RW) {
         __syncwarp();  // the own row of P
@@ -405,8 +414,9 @@ __device__ __forceinline__ void resident_tile(Smem<TY>& sm, const Job& b, const 
   }
 }
 
-template <int SF, int TY>
-__global__ void __launch_bounds__(threads_of(TY), TY == 4 ? 5 : 6)
+// OCC: CTAs per SM the registers are sized for (few_ctas and more_ctas below).
+template <int SF, int TY, int OCC>
+__global__ void __launch_bounds__(threads_of(TY), OCC)
     k_resident(const float4* Qs, float4* Qo, const float4* __restrict__ Mi, const float4* __restrict__ Mj, float* dt,
                uint32_t* wave, ExHead* ex, const int nsteps, const int first, const int last, float* out, int* out_err, int* err, const Consts c,
                const int M, const int N) {
@@ -418,8 +428,8 @@ __global__ void __launch_bounds__(threads_of(TY), TY == 4 ? 5 : 6)
 // All solves of a batch in one launch: items[blockIdx.x] is a solve and one of its tiles.
 // The schemes are separate bodies, chosen once per CTA, so that the registers are those
 // of the largest one.
-template <int TY>
-__global__ void __launch_bounds__(threads_of(TY), TY == 4 ? 5 : 6)
+template <int TY, int OCC>
+__global__ void __launch_bounds__(threads_of(TY), OCC)
     k_resident_batch(const BatchSolve* __restrict__ solves, const int2* __restrict__ items, ExHead* ex,
                      const int nsolves, const int nsteps, const int first, const int last, int* err) {
   __shared__ Smem<TY> sm;
@@ -455,17 +465,27 @@ int resident_ctas(const void* kern, int threads) {
 
 using Kern = void (*)(const float4*, float4*, const float4*, const float4*, float*, uint32_t*, ExHead*, int, int, int,
                       float*, int*, int*, Consts, int, int);
-template <int TY> Kern kernel_of(int sf) {
+template <int TY, int OCC> Kern kernel_of(int sf) {
   switch (sf) {
-    case 0: return k_resident<0, TY>;
-    case 1: return k_resident<1, TY>;
-    case 2: return k_resident<2, TY>;
-    case 4: return k_resident<4, TY>;
-    case 5: return k_resident<5, TY>;
-    default: return k_resident<6, TY>;
+    case 0: return k_resident<0, TY, OCC>;
+    case 1: return k_resident<1, TY, OCC>;
+    case 2: return k_resident<2, TY, OCC>;
+    case 4: return k_resident<4, TY, OCC>;
+    case 5: return k_resident<5, TY, OCC>;
+    default: return k_resident<6, TY, OCC>;
   }
 }
-Kern kernel_of(int sf, int rows) { return rows == 4 ? kernel_of<4>(sf) : kernel_of<8>(sf); }
+// Tiles of height TY a launch can take, by the kernels built for OCC CTAs per SM (every
+// scheme's is built for the same).
+template <int TY, int OCC> int capacity() {
+  static const int n = std::min(resident_ctas((const void*)k_resident<4, TY, OCC>, threads_of(TY)),
+                                resident_ctas((const void*)k_resident_batch<TY, OCC>, threads_of(TY)));
+  return n;
+}
+template <int TY> bool few(int tiles) { return tiles <= capacity<TY, few_ctas(TY)>(); }
+template <int TY> Kern kernel_of(int sf, int tiles) {
+  return few<TY>(tiles) ? kernel_of<TY, few_ctas(TY)>(sf) : kernel_of<TY, more_ctas(TY)>(sf);
+}
 
 }  // namespace
 
@@ -475,13 +495,8 @@ int resident_tiles(int M, int N, int rows) { return rows == 4 ? tiles_of<4>(M, N
 // lower tiles have the shorter stage at every size that fits (table above).  8 rows up to
 // 888 tiles (227 K cells); beyond, a CTA would have to work on several tiles in turn.
 int resident_rows(int tiles4, int tiles8) {
-  // every instantiation of a height is built for the same occupancy
-  static const int cap4 = std::min(resident_ctas((const void*)k_resident<4, 4>, threads_of(4)),
-                                   resident_ctas((const void*)k_resident_batch<4>, threads_of(4)));
-  static const int cap8 = std::min(resident_ctas((const void*)k_resident<4, 8>, threads_of(8)),
-                                   resident_ctas((const void*)k_resident_batch<8>, threads_of(8)));
-  if (tiles4 <= cap4 && tiles4 <= kMaxTiles4) return 4;
-  return tiles8 <= cap8 && tiles8 <= kMaxTiles8 ? 8 : 0;
+  if (tiles4 <= std::min(capacity<4, more_ctas(4)>(), kMaxTiles4)) return 4;
+  return tiles8 <= std::min(capacity<8, more_ctas(8)>(), kMaxTiles8) ? 8 : 0;
 }
 
 // ---- exchange buffers ----
@@ -592,17 +607,19 @@ void resident_user(int dev, int change) {
 cudaError_t launch_resident(int scheme, const float4* Qs, float4* Qo, const float4* Mi, const float4* Mj, float* dt,
                             uint32_t* wave, int rows, int nsteps, bool first, bool last, float* out, int* out_err,
                             int* err, const Consts& c, int M, int N, cudaStream_t s) {
+  const int sf = scheme + (c.muscl > 0 ? 4 : 0), tiles = resident_tiles(M, N, rows);
   return with_buffer(s, [&](ExHead* ex) {
-    return launch_coop(kernel_of(scheme + (c.muscl > 0 ? 4 : 0), rows), resident_tiles(M, N, rows), threads_of(rows), s,
-                       Qs, Qo, Mi, Mj, dt, wave, ex, nsteps, (int)first, (int)last, out, out_err, err, c, M, N);
+    return launch_coop(rows == 4 ? kernel_of<4>(sf, tiles) : kernel_of<8>(sf, tiles), tiles, threads_of(rows), s, Qs,
+                       Qo, Mi, Mj, dt, wave, ex, nsteps, (int)first, (int)last, out, out_err, err, c, M, N);
   });
 }
 
 cudaError_t launch_resident_batch(const BatchSolve* solves, const int2* items, int tiles, int rows, int nsolves,
                                   int nsteps, bool first, bool last, int* err, cudaStream_t s) {
   return with_buffer(s, [&](ExHead* ex) {
-    return launch_coop(rows == 4 ? k_resident_batch<4> : k_resident_batch<8>, tiles, threads_of(rows), s, solves, items,
-                       ex, nsolves, nsteps, (int)first, (int)last, err);
+    auto k = rows == 4 ? (few<4>(tiles) ? k_resident_batch<4, few_ctas(4)> : k_resident_batch<4, more_ctas(4)>)
+                       : (few<8>(tiles) ? k_resident_batch<8, few_ctas(8)> : k_resident_batch<8, more_ctas(8)>);
+    return launch_coop(k, tiles, threads_of(rows), s, solves, items, ex, nsolves, nsteps, (int)first, (int)last, err);
   });
 }
 
