@@ -79,7 +79,8 @@ __global__ void __launch_bounds__(256)
     k_ex_fluxes(const V4<R>* __restrict__ st, const V2<R>* __restrict__ V, V4<R>* __restrict__ fx,
                  V4<R>* __restrict__ fy, const ConstsR<R> c, int M, int N) {
   __shared__ V4<R> P[11][35];
-  const int tx = threadIdx.x, ty = threadIdx.y, i0 = blockIdx.x * 32, j0 = blockIdx.y * 8;
+  const int tx = threadIdx.x, ty = threadIdx.y, across = (M + 31) / 32;  // blocks row by row
+  const int i0 = (int)(blockIdx.x % across) * 32, j0 = (int)(blockIdx.x / across) * 8;
   const int i = i0 + tx, j = j0 + ty;
   const bool jf = i < M && j <= N, jn = i < M && j < N;
   R nx = 0, ny = 0, mx = 0, my = 0, len;
@@ -231,7 +232,7 @@ inline int grid1d(size_t n) { return (int)std::min<size_t>((n + 255) / 256, 148 
 template <int SCHEME>
 void fluxes(const V4<R>* st, const V2<R>* V, V4<R>* fx, V4<R>* fy, const ConstsR<R>& c, int M, int N,
             cudaStream_t s) {
-  launch_pdl(k_ex_fluxes<SCHEME>, dim3((M + 31) / 32, (N + 8) / 8), dim3(32, 8), 0, s, st, V, fx, fy, c, M, N);
+  launch_pdl(k_ex_fluxes<SCHEME>, dim3((M + 31) / 32 * ((N + 8) / 8)), dim3(32, 8), 0, s, st, V, fx, fy, c, M, N);
 }
 
 }  // namespace

@@ -78,7 +78,8 @@ __global__ void __launch_bounds__(256)
     k_ref_fluxes(const float4* __restrict__ st, const float2* __restrict__ V, float4* __restrict__ fx,
                  float4* __restrict__ fy, const Consts c, int M, int N) {
   __shared__ float4 P[11][35];
-  const int tx = threadIdx.x, ty = threadIdx.y, i0 = blockIdx.x * 32, j0 = blockIdx.y * 8;
+  const int tx = threadIdx.x, ty = threadIdx.y, across = (M + 31) / 32;  // blocks row by row
+  const int i0 = (int)(blockIdx.x % across) * 32, j0 = (int)(blockIdx.x / across) * 8;
   const int i = i0 + tx, j = j0 + ty;
   const bool jf = i < M && j <= N, jn = i < M && j < N;
   float nx = 0, ny = 0, mx = 0, my = 0, len;
@@ -184,7 +185,7 @@ void launch_ref_boundary(const float4* in, float4* out, const float2* V, const C
 }
 void launch_ref_fluxes(int scheme, const float4* st, const float2* V, float4* fx, float4* fy, const Consts& c, int M,
                        int N, cudaStream_t s) {
-  const dim3 g((M + 31) / 32, (N + 8) / 8), b(32, 8);
+  const dim3 g((M + 31) / 32 * ((N + 8) / 8)), b(32, 8);
   if (scheme == 0) launch_pdl(k_ref_fluxes<0>, g, b, 0, s, st, V, fx, fy, c, M, N);
   else if (scheme == 1) launch_pdl(k_ref_fluxes<1>, g, b, 0, s, st, V, fx, fy, c, M, N);
   else launch_pdl(k_ref_fluxes<2>, g, b, 0, s, st, V, fx, fy, c, M, N);
