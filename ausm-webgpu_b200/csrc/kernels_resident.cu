@@ -528,8 +528,12 @@ cudaError_t take(Pool& pool, cudaStream_t s, Buffer** out) {
   for (Buffer& b : pool.buffers)
     if (b.stream == s) best = &b;
   if (!best)
-    for (Buffer& b : pool.buffers)
-      if (!best && cudaEventQuery(b.done) == cudaSuccess) best = &b;
+    for (Buffer& b : pool.buffers) {
+      if (best) break;
+      const cudaError_t e = cudaEventQuery(b.done);
+      if (e == cudaSuccess) best = &b;
+      else if (e == cudaErrorNotReady) cudaGetLastError();  // not an error of this thread's calls
+    }
   if (!best && (int)pool.buffers.size() < kMaxBuffers) {
     Buffer b;
     cudaError_t e = cudaMalloc((void**)&b.p, kExBytes);
