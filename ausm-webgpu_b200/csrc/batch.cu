@@ -61,6 +61,7 @@ struct ausm_batch {
   std::vector<int2> ritems;       // their work items (the device's d_ritems)
   int2* d_ritems = nullptr;
   int ritem_cap = 0;
+  bool res_stepped = false;       // a direct (resident) step has run: see tune_rows
   int tuned_rows = 0;             // height chosen by the last tuning run (0: none yet)
   double tuned_cells = 0.0;       // the batch's cell count at that run
   int* d_err = nullptr;           // set by a TMA tile whose bounded wait gave up
@@ -333,8 +334,11 @@ void enqueue_steps(ausm_batch* b, int n) {
 // candidate height the work list is laid out again and the stage-1 launches of every
 // scheme group are timed on the members' own data (stage 1 writes only each member's
 // scratch buffer).  Runs on the first step and again when the batch's cell count has
-// changed by more than a factor of two; AUSM_TILE_ROWS fixes the height.
-int tune_rows(ausm_batch* b) {
+// changed by more than a factor of two; AUSM_TILE_ROWS fixes the height.  It times and
+// waits, which a stream capture does not allow: a captured step needs a direct one before
+// it.  Where direct steps are resident they tune nothing, and a captured step takes the
+// height in use (16 rows if none has been tuned).
+int tune_rows(ausm_batch* b, bool captured) {
   double cells = 0.0;
   for (ausm_solver* h : b->members) cells += (double)h->M * h->N;
   if (!b->tma) return AUSM_OK;
@@ -352,6 +356,7 @@ int tune_rows(ausm_batch* b) {
     return AUSM_OK;
   }
   if (b->tuned_rows && cells <= 2.0 * b->tuned_cells && 2.0 * cells >= b->tuned_cells) return AUSM_OK;
+  if (captured && b->res_rows && b->res_stepped) return AUSM_OK;
   const int reps = (int)std::max(5.0, std::min(100.0, 1.0e8 / std::max(cells, 1.0)));
   float best_ms[3] = {INFINITY, INFINITY, INFINITY};
   const int cand[3] = {8, 16, 32};
@@ -586,14 +591,20 @@ int batch_step_impl(ausm_batch* b, int n, float* dt_wave, bool read_err) {
   if (ns == 0 || n == 0) return AUSM_OK;
   for (ausm_solver* h : b->members)
     BNEED(b, h->has_grid && h->has_state, AUSM_ERR_STATE, "a member lost its grid or state");
-  // members whose tiles all fit on the chip together step in one launch
-  bool resident = !ausm::forced_tile_rows() && b->res_rows != 0, refused = false;
+  // Members whose tiles all fit on the chip together step in one launch; a host's stream
+  // capture stays on the stage kernels: a captured launch would hold an exchange buffer
+  // that others use.
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  BCU(b, cudaStreamIsCapturing(b->st, &cap));
+  const bool captured = cap != cudaStreamCaptureStatusNone;
+  bool resident = !ausm::forced_tile_rows() && b->res_rows != 0 && !captured, refused = false;
   if (resident) {
     if ((rc = sync_descriptors(b)) || (rc = resident_steps(b, n, &refused))) return rc;
     resident = !refused;
+    if (resident) b->res_stepped = true;
   }
   if (!resident) {
-    if ((rc = tune_rows(b)) || (rc = sync_descriptors(b)) || (rc = run_steps(b, n))) return rc;
+    if ((rc = tune_rows(b, captured)) || (rc = sync_descriptors(b)) || (rc = run_steps(b, n))) return rc;
   }
   for (size_t k = 0; k < b->members.size(); k++) {
     ausm_solver* h = b->members[b->order[k]];

@@ -530,9 +530,8 @@ cudaError_t take(Pool& pool, cudaStream_t s, Buffer** out) {
   if (!best)
     for (Buffer& b : pool.buffers) {
       if (best) break;
-      const cudaError_t e = cudaEventQuery(b.done);
-      if (e == cudaSuccess) best = &b;
-      else if (e == cudaErrorNotReady) cudaGetLastError();  // not an error of this thread's calls
+      if (cudaEventQuery(b.done) == cudaSuccess) best = &b;
+      else cudaGetLastError();  // busy, or not to be asked now: not an error of this thread's calls
     }
   if (!best && (int)pool.buffers.size() < kMaxBuffers) {
     Buffer b;

@@ -1,0 +1,91 @@
+"""Steps captured into a CUDA graph of the host's own.  A captured step stays on the stage
+kernels at any size: a captured resident launch would hold an exchange buffer that other
+solvers use between the replays.  Replays beside another solver's direct steps, and direct
+steps after them, must give the bits of a twin that is stepped directly throughout, for a
+single solve and for a batch (graphs off), both small enough that their direct steps are
+resident."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from test_gpu_edges import solver
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(96, 40, "SLAU2"), (65, 33, "AUSM+-up"), (33, 17, "SLAU")]
+
+
+class Graph:
+    """What fn enqueues on a stream, captured and replayed through the driver API."""
+
+    def __init__(self, stream, fn):
+        self.cu, self.stream = C.CDLL("libcuda.so.1"), stream
+        g, self.exec = C.c_void_p(), C.c_void_p()
+        self.ok(self.cu.cuStreamBeginCapture_v2(stream, 1))  # thread-local
+        fn()
+        self.ok(self.cu.cuStreamEndCapture(stream, C.byref(g)))
+        self.ok(self.cu.cuGraphInstantiateWithFlags(C.byref(self.exec), g, C.c_ulonglong(0)))
+        self.ok(self.cu.cuGraphDestroy(g))
+
+    def ok(self, rc):
+        assert rc == 0, f"CUDA driver error {rc}"
+
+    def launch(self):
+        self.ok(self.cu.cuGraphLaunch(self.exec, self.stream))
+
+    def close(self):
+        self.ok(self.cu.cuGraphExecDestroy(self.exec))
+
+
+def stream_of(s):
+    from ausm import _lib
+    st = C.c_void_p()
+    s._c(_lib.lib().ausm_stream(s.h, C.byref(st)))
+    return st
+
+
+def test_captured_solver_step_beside_direct_steps():
+    a, twin, other, other_twin = (solver(*x) for x in ((96, 40), (96, 40), (257, 131), (257, 131)))
+    for s in (a, twin):
+        s.step(3)
+    g = Graph(stream_of(a), lambda: a.step(3, wait=False))
+    for _ in range(5):
+        g.launch()
+        other.step(30, wait=False)
+        twin.step(3)
+        other_twin.step(30)
+    for s in (a, twin, other, other_twin):
+        s.step(4)
+    g.close()
+    for x, y in ((a, twin), (other, other_twin)):
+        assert x.max_wave_speed() == y.max_wave_speed()
+        np.testing.assert_array_equal(x.state(), y.state())
+    for s in (a, twin, other, other_twin):
+        s.close()
+
+
+def test_captured_batch_step_beside_direct_steps():
+    from ausm import Batch
+    mine, twins = ([solver(M, N, scheme=sc) for M, N, sc in SIZES] for _ in range(2))
+    other, other_twin = solver(257, 131), solver(257, 131)
+    with Batch(graphs=False) as b, Batch(graphs=False) as t:
+        for s, x in zip(mine, twins):
+            b.add(s)
+            t.add(x)
+        np.testing.assert_array_equal(b.step(3), t.step(3))
+        g = Graph(stream_of(mine[0]), lambda: b.step(3, wait=False))
+        other.step(30, wait=False)  # whatever the capture left behind is not this solver's error
+        other_twin.step(30)
+        for _ in range(5):
+            g.launch()
+            other.step(30, wait=False)
+            t.step(3)
+            other_twin.step(30)
+        np.testing.assert_array_equal(b.step(4), t.step(4))
+        b.synchronize()
+        g.close()
+    for x, y in zip(mine + [other], twins + [other_twin]):
+        np.testing.assert_array_equal(x.state(), y.state())
+    for s in mine + twins + [other, other_twin]:
+        s.close()
