@@ -13,6 +13,9 @@
 // arithmetic (72 operations a vertex at half rate, halo and idle lanes included) and the
 // tiles' way in and out of L2, which all CTAs of the launch take at the same time; on
 // small grids the latency of the colour steps, 0.4 us each.
+#include <mutex>
+#include <set>
+
 #include "ausm_internal.h"
 #include "tma.cuh"
 
@@ -272,18 +275,28 @@ dim3 grid_tiles(int M, int N, int halo, int max_h) {
   const int rounds = (nx * need + kSMs - 1) / kSMs;
   return dim3(nx, std::max(need, std::min(std::max(1, kSMs * rounds / nx), N - 1)));
 }
-template <class K, class... Args>
-void launch_sweeps(K kern, dim3 tiles, int threads, size_t smem, cudaStream_t s, Args... args) {
-  if (smem > 46 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  launch_pdl(kern, tiles, dim3(threads), smem, s, args...);
+// Lets KERN take `bytes`, what its largest tile needs, on the current device: once per
+// device and before its first launch there.  The limit belongs to the kernel and is shared
+// by all host threads; set per launch to the launch's own size, it changed under another
+// thread's launch, and grids of two sizes generated at once came out wrong.
+template <auto KERN> void allow_smem(int bytes) {
+  static std::mutex mu;
+  static std::set<int> done;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(mu);
+  if (done.count(dev)) return;
+  if (cudaFuncSetAttribute(KERN, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess) done.insert(dev);
 }
-template <int NC, int S, int NW>
+template <int NC, int S, int NW, int MAX_H>
 void sweeps_d(const double2* src, double2* dst, const double2* ends, int M, int N, int sweeps, double omega,
-              uint32_t* move, int max_h, cudaStream_t s) {
-  const dim3 g = grid_tiles(M, N, NC * S, max_h);
+              uint32_t* move, cudaStream_t s) {
+  constexpr int ROW = GW * (int)sizeof(double2);
+  const dim3 g = grid_tiles(M, N, NC * S, MAX_H);
   const int h = (N - 1 + g.y - 1) / g.y;
-  launch_sweeps(k_grid_multicolor<NC, S, NW>, g, 32 * NW, (size_t)(h + 2 * NC * S) * GW * sizeof(double2), s, src, dst,
-                ends, M, N, sweeps, omega, move);
+  constexpr auto kern = k_grid_multicolor<NC, S, NW>;
+  allow_smem<kern>((MAX_H + 2 * NC * S) * ROW);
+  launch_pdl(kern, g, dim3(32 * NW), (size_t)(h + 2 * NC * S) * ROW, s, src, dst, ends, M, N, sweeps, omega, move);
 }
 // Two sweeps to a launch while the tiles of that halo (48 or 40 columns, up to 32 rows) fit
 // the SMs one each: there a launch is bound by its fixed cost and the latency of the colour
@@ -308,22 +321,23 @@ void launch_grid_init_d(double2* V, int M, int N, double first_spacing, cudaStre
 constexpr int kJacobiSweeps = 6;
 int grid_jacobi_sweeps() { return kJacobiSweeps; }
 void launch_grid_jacobi(const float2* src, float2* dst, const float2* ends, int M, int N, int sweeps, cudaStream_t s) {
-  constexpr int NW = 16;
-  const dim3 g = grid_tiles(M, N, kJacobiSweeps, 48);
+  constexpr int NW = 16, MAX_H = 48, ROW = 2 * GW * (int)sizeof(float2);
+  const dim3 g = grid_tiles(M, N, kJacobiSweeps, MAX_H);
   const int h = (N - 1 + g.y - 1) / g.y;
-  launch_sweeps(k_grid_jacobi<kJacobiSweeps, NW>, g, 32 * NW, 2 * (size_t)(h + 2 * kJacobiSweeps) * GW * sizeof(float2), s,
-                src, dst, ends, M, N, sweeps);
+  constexpr auto kern = k_grid_jacobi<kJacobiSweeps, NW>;
+  allow_smem<kern>((MAX_H + 2 * kJacobiSweeps) * ROW);
+  launch_pdl(kern, g, dim3(32 * NW), (size_t)(h + 2 * kJacobiSweeps) * ROW, s, src, dst, ends, M, N, sweeps);
 }
 
 int grid_multicolor_sweeps(int M, int N) { return two_sweeps(M, N) ? 2 : 1; }
 void launch_grid_multicolor_d(const double2* src, double2* dst, const double2* ends, int M, int N, int sweeps,
                               double omega, uint32_t* move, cudaStream_t s) {
   if (two_sweeps(M, N)) {
-    if (M & 1) sweeps_d<6, 2, 16>(src, dst, ends, M, N, sweeps, omega, move, 32, s);
-    else sweeps_d<4, 2, 16>(src, dst, ends, M, N, sweeps, omega, move, 32, s);
+    if (M & 1) sweeps_d<6, 2, 16, 32>(src, dst, ends, M, N, sweeps, omega, move, s);
+    else sweeps_d<4, 2, 16, 32>(src, dst, ends, M, N, sweeps, omega, move, s);
   } else {
-    if (M & 1) sweeps_d<6, 1, 8>(src, dst, ends, M, N, sweeps, omega, move, 40, s);
-    else sweeps_d<4, 1, 8>(src, dst, ends, M, N, sweeps, omega, move, 40, s);
+    if (M & 1) sweeps_d<6, 1, 8, 40>(src, dst, ends, M, N, sweeps, omega, move, s);
+    else sweeps_d<4, 1, 8, 40>(src, dst, ends, M, N, sweeps, omega, move, s);
   }
 }
 
