@@ -1060,6 +1060,13 @@ int ausm_debug_set_wait_polls(unsigned polls) {
   return AUSM_OK;
 }
 
+int ausm_debug_set_exchange_tag(unsigned tag) {
+  int dev = 0;
+  CU((ausm_solver*)nullptr, cudaGetDevice(&dev));
+  set_exchange_tag(dev, tag);
+  return AUSM_OK;
+}
+
 int ausm_autotune(ausm_solver* h, int force, int* rows) {
   NEED(h, h, AUSM_ERR_INVALID, "null handle");
   NEED(h, h->has_grid && h->has_state, AUSM_ERR_STATE, "need a grid and a state");

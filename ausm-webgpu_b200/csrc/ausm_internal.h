@@ -211,9 +211,11 @@ cudaError_t launch_resident(int scheme, const float4* Qs, float4* Qo, const floa
                             int* err, const Consts& c, int M, int N, cudaStream_t s);
 // The same for a batch: items[k] = (descriptor, tile of that solve); every solve goes from
 // Q[cur] to Q[(cur + nsteps) % 3].
-cudaError_t launch_resident_batch(const BatchSolve* solves, const int2* items, int tiles, int rows, int nsolves,
-                                  int nsteps, bool first, bool last, int* err, cudaStream_t s);
+cudaError_t launch_resident_batch(const BatchSolve* solves, const int2* items, int tiles, int rows, int nsteps,
+                                  bool first, bool last, int* err, cudaStream_t s);
 cudaError_t set_wait_polls_resident(unsigned polls);
+// Test hook: the next tag of every exchange buffer the device has (at least 1).
+void set_exchange_tag(int dev, uint32_t tag);
 // Counts the solvers and batches of a device (+1, -1); with the last one its exchange
 // buffers are freed.
 void resident_user(int dev, int change);

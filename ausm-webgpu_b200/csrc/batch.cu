@@ -424,7 +424,7 @@ int resident_steps(ausm_batch* b, int n, bool* refused) {
   for (int done = 0; done < n;) {
     const int k = std::min(n - done, ausm::kResidentSteps);
     const cudaError_t e =
-        ausm::launch_resident_batch(b->d_solves, b->d_ritems, (int)b->ritems.size(), b->res_rows, ns, k, done == 0,
+        ausm::launch_resident_batch(b->d_solves, b->d_ritems, (int)b->ritems.size(), b->res_rows, k, done == 0,
                                     done + k == n, b->d_err, b->st);
     if (done == 0 && e == cudaErrorCooperativeLaunchTooLarge) {
       cudaGetLastError();

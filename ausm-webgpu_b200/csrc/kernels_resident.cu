@@ -19,8 +19,10 @@
 // 8-byte accesses are single-copy atomic, so a word is never half old.  Two copies of
 // the buffer, by the parity of the tag: a tile writes stage s + 2 only after it has read
 // its neighbours' stage s + 1, which they wrote after reading this tile's stage s, so a
-// word is never overwritten before it has been read.  Tags go on from launch to launch,
-// counted in the buffer's header, so whoever uses a buffer next finds no tag of its own.
+// word is never overwritten before it has been read.  Tags go on from launch to launch of
+// a buffer, counted on the host, and a buffer is cleared before they would wrap (after 2^32
+// stages, an hour and a half of the smallest grids): so whoever uses it next finds none of
+// its own tags in cells that only larger launches write.
 //
 // Every wait is bounded (c_wait_polls); a CTA that gives up sets *err and returns, and
 // the others see *err in their own waits.
@@ -125,13 +127,6 @@ template <int TY> struct Smem {
   float4 Qn[TY][TX];          // state at the start of the step
 };
 
-// Head of an exchange buffer; the tiles' cells follow.
-struct ExHead {
-  uint32_t tag;     // of the first exchange of the next launch
-  uint32_t solves;  // finished solves of the running launch
-  uint32_t pad[62];
-};
-
 // What a CTA of the launch works on (one tile of one solve).
 struct Job {
   const float4* Qs;
@@ -145,9 +140,10 @@ struct Job {
   int M, N, t;     // t: tile of the solve
 };
 
+// ex: the solve's tiles in the exchange buffer; tag0: tag of the state before the first stage.
 template <int SF, int TY>
-__device__ __forceinline__ void resident_tile(Smem<TY>& sm, const Job& b, const Consts& c, ExHead* head, int tile0,
-                                              int nsolves, int nsteps, bool first, bool last, int* err) {
+__device__ __forceinline__ void resident_tile(Smem<TY>& sm, const Job& b, const Consts& c, ulonglong2* ex, const uint32_t tag0, int nsteps,
+                                              bool first, bool last, int* err) {
   using E = Ex<TY>;
   constexpr int CPT = TY / RW;
   constexpr bool EARLY = TY == 4;
@@ -176,11 +172,9 @@ __device__ __forceinline__ void resident_tile(Smem<TY>& sm, const Job& b, const 
     nb = sel < 2 ? (q.tx == 0 ? b.t + q.nx - 1 : b.t - 1) : (q.tx == q.nx - 1 ? b.t - q.nx + 1 : b.t + 1);
     cell = (sel < 2 ? E::RIGHT + TY * sel : E::LEFT + TY * (sel - 2)) + r;
   }
-  ulonglong2* const ex = reinterpret_cast<ulonglong2*>(head + 1) + (size_t)tile0 * E::TILE;  // the solve's tiles
   const ulonglong2* const from = ex + (fetch ? (size_t)nb * E::TILE + cell : 0);
   float4* const halo = &sm.P[0][0] + (fetch ? pr * (TX + 4) + pc : 0);
   ulonglong2* mine = ex + (size_t)b.t * E::TILE;
-  const uint32_t tag0 = *(volatile uint32_t*)&head->tag;  // of the state before the first stage
   // The first stage's halo comes from the state itself, except when the launch writes its
   // result over that state: then it is exchanged like any other, so that no tile reads
   // cells that another one writes.
@@ -384,10 +378,9 @@ __device__ __forceinline__ void resident_tile(Smem<TY>& sm, const Job& b, const 
       }
     }
   }
-  // Every tile of the solve has read wave[0] and the tag by the time the last one gets
-  // here; that one publishes the max wave speed of the new state, and the last tile of the
-  // last solve moves the tag on.  Accumulator and counts are zero again for the next
-  // launch, also when a wait gave up.
+  // Every tile of the solve has read wave[0] by the time the last one gets here; that one
+  // publishes the max wave speed of the new state.  Accumulator and count are zero again for
+  // the next launch, also when a wait gave up.
   if (last) block_max_to(&b.wave[1], wmax);
   if (tid == 0) {
     __threadfence();
@@ -405,11 +398,6 @@ __device__ __forceinline__ void resident_tile(Smem<TY>& sm, const Job& b, const 
         }
       }
       if (b.out_err) *b.out_err = e;
-      __threadfence();
-      if (atomicAdd(&head->solves, 1u) == (uint32_t)nsolves - 1) {
-        head->solves = 0u;
-        head->tag = tag0 + (uint32_t)stages;
-      }
     }
   }
 }
@@ -418,11 +406,11 @@ __device__ __forceinline__ void resident_tile(Smem<TY>& sm, const Job& b, const 
 template <int SF, int TY, int OCC>
 __global__ void __launch_bounds__(threads_of(TY), OCC)
     k_resident(const float4* Qs, float4* Qo, const float4* __restrict__ Mi, const float4* __restrict__ Mj, float* dt,
-               uint32_t* wave, ExHead* ex, const int nsteps, const int first, const int last, float* out, int* out_err, int* err, const Consts c,
+               uint32_t* wave, ulonglong2* ex, const uint32_t tag0, const int nsteps, const int first, const int last, float* out, int* out_err, int* err, const Consts c,
                const int M, const int N) {
   __shared__ Smem<TY> sm;
   const Job b = {Qs, Qo, Mi, Mj, dt, wave, out, out_err, M, N, (int)blockIdx.x};
-  resident_tile<SF, TY>(sm, b, c, ex, 0, 1, nsteps, first != 0, last != 0, err);
+  resident_tile<SF, TY>(sm, b, c, ex, tag0, nsteps, first != 0, last != 0, err);
 }
 
 // All solves of a batch in one launch: items[blockIdx.x] is a solve and one of its tiles.
@@ -430,15 +418,16 @@ __global__ void __launch_bounds__(threads_of(TY), OCC)
 // of the largest one.
 template <int TY, int OCC>
 __global__ void __launch_bounds__(threads_of(TY), OCC)
-    k_resident_batch(const BatchSolve* __restrict__ solves, const int2* __restrict__ items, ExHead* ex,
-                     const int nsolves, const int nsteps, const int first, const int last, int* err) {
+    k_resident_batch(const BatchSolve* __restrict__ solves, const int2* __restrict__ items, ulonglong2* ex,
+                     const uint32_t tag0, const int nsteps, const int first, const int last, int* err) {
   __shared__ Smem<TY> sm;
   const int2 it = items[blockIdx.x];
   const BatchSolve& d = solves[it.x];
   const Consts c = d.c;
   const Job b = {d.Q[d.cur], d.Q[(d.cur + nsteps) % 3], d.Mi, d.Mj, d.dt, d.wave, nullptr, nullptr, d.M, d.N, it.y};
   auto go = [&](auto sf) {
-    resident_tile<decltype(sf)::value, TY>(sm, b, c, ex, d.rtile0, nsolves, nsteps, first != 0, last != 0, err);
+    resident_tile<decltype(sf)::value, TY>(sm, b, c, ex + (size_t)d.rtile0 * Ex<TY>::TILE, tag0, nsteps, first != 0,
+                                           last != 0, err);
   };
   switch (d.scheme) {
     case 0: go(std::integral_constant<int, 0>()); break;
@@ -463,8 +452,8 @@ int resident_ctas(const void* kern, int threads) {
   return sms * per;
 }
 
-using Kern = void (*)(const float4*, float4*, const float4*, const float4*, float*, uint32_t*, ExHead*, int, int, int,
-                      float*, int*, int*, Consts, int, int);
+using Kern = void (*)(const float4*, float4*, const float4*, const float4*, float*, uint32_t*, ulonglong2*, uint32_t, int,
+                      int, int, float*, int*, int*, Consts, int, int);
 template <int TY, int OCC> Kern kernel_of(int sf) {
   switch (sf) {
     case 0: return k_resident<0, TY, OCC>;
@@ -507,9 +496,10 @@ int resident_rows(int tiles4, int tiles8) {
 // (on the device) for the oldest.
 namespace {
 constexpr int kMaxBuffers = 8;
-constexpr size_t kExBytes = sizeof(ExHead) + 16 * std::max(kMaxTiles4 * Ex<4>::TILE, kMaxTiles8 * Ex<8>::TILE);
+constexpr size_t kExBytes = 16 * std::max(kMaxTiles4 * Ex<4>::TILE, kMaxTiles8 * Ex<8>::TILE);
 struct Buffer {
-  ExHead* p = nullptr;
+  ulonglong2* p = nullptr;
+  uint32_t tag = 1;  // of the next launch's first exchange; 0 is that of a cleared buffer
   cudaEvent_t done = nullptr;
   cudaStream_t stream = nullptr;
   uint64_t used = 0;
@@ -522,8 +512,8 @@ struct Pool {
 std::mutex g_pool_mu;
 std::map<int, Pool> g_pool;  // per device
 
-// With g_pool_mu held and the device current.
-cudaError_t take(Pool& pool, cudaStream_t s, Buffer** out) {
+// A buffer for a launch of `stages` stages on s.  With g_pool_mu held and the device current.
+cudaError_t take(Pool& pool, cudaStream_t s, uint32_t stages, Buffer** out) {
   Buffer* best = nullptr;
   for (Buffer& b : pool.buffers)
     if (b.stream == s) best = &b;
@@ -538,7 +528,6 @@ cudaError_t take(Pool& pool, cudaStream_t s, Buffer** out) {
     cudaError_t e = cudaMalloc((void**)&b.p, kExBytes);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaMemsetAsync(b.p, 0, kExBytes, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(&b.p->tag, 1, sizeof(uint32_t), s);  // no tag of a zeroed buffer
     if (e != cudaSuccess) {
       if (b.done) cudaEventDestroy(b.done);
       if (b.p) cudaFree(b.p);
@@ -554,6 +543,11 @@ cudaError_t take(Pool& pool, cudaStream_t s, Buffer** out) {
   }
   best->stream = s;
   best->used = ++pool.clock;
+  if (best->tag > UINT32_MAX - stages) {  // the tags would wrap: start again on a cleared buffer
+    const cudaError_t e = cudaMemsetAsync(best->p, 0, kExBytes, s);
+    if (e != cudaSuccess) return e;
+    best->tag = 1;
+  }
   *out = best;
   return cudaSuccess;
 }
@@ -572,9 +566,10 @@ cudaError_t launch_coop(void (*kern)(KArgs...), int ctas, int threads, cudaStrea
   return cudaLaunchKernelEx(&cfg, kern, static_cast<Args&&>(args)...);
 }
 
-// Takes a buffer of the current device for s, calls launch(buffer), notes when it is free.
-// None of it belongs to a stream capture another thread may have open.
-template <class F> cudaError_t with_buffer(cudaStream_t s, F launch) {
+// Takes a buffer of the current device for `nsteps` steps on s, calls launch(cells, first
+// tag), notes when the buffer is free.  None of it belongs to a stream capture another
+// thread may have open.
+template <class F> cudaError_t with_buffer(cudaStream_t s, int nsteps, F launch) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -583,9 +578,10 @@ template <class F> cudaError_t with_buffer(cudaStream_t s, F launch) {
   {
     std::lock_guard<std::mutex> lk(g_pool_mu);
     Buffer* b = nullptr;
-    e = take(g_pool[dev], s, &b);
+    e = take(g_pool[dev], s, 3u * nsteps, &b);
     if (e == cudaSuccess) {
-      e = launch(b->p);
+      e = launch(b->p, b->tag);
+      if (e == cudaSuccess) b->tag += 3u * nsteps;
       const cudaError_t e2 = cudaEventRecord(b->done, s);
       if (e == cudaSuccess) e = e2;
     }
@@ -594,6 +590,11 @@ template <class F> cudaError_t with_buffer(cudaStream_t s, F launch) {
   return e;
 }
 }  // namespace
+
+void set_exchange_tag(int dev, uint32_t tag) {
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  for (Buffer& b : g_pool[dev].buffers) b.tag = std::max(tag, 1u);
+}
 
 void resident_user(int dev, int change) {
   std::lock_guard<std::mutex> lk(g_pool_mu);
@@ -611,18 +612,18 @@ cudaError_t launch_resident(int scheme, const float4* Qs, float4* Qo, const floa
                             uint32_t* wave, int rows, int nsteps, bool first, bool last, float* out, int* out_err,
                             int* err, const Consts& c, int M, int N, cudaStream_t s) {
   const int sf = scheme + (c.muscl > 0 ? 4 : 0), tiles = resident_tiles(M, N, rows);
-  return with_buffer(s, [&](ExHead* ex) {
+  return with_buffer(s, nsteps, [&](ulonglong2* ex, uint32_t tag0) {
     return launch_coop(rows == 4 ? kernel_of<4>(sf, tiles) : kernel_of<8>(sf, tiles), tiles, threads_of(rows), s, Qs,
-                       Qo, Mi, Mj, dt, wave, ex, nsteps, (int)first, (int)last, out, out_err, err, c, M, N);
+                       Qo, Mi, Mj, dt, wave, ex, tag0, nsteps, (int)first, (int)last, out, out_err, err, c, M, N);
   });
 }
 
-cudaError_t launch_resident_batch(const BatchSolve* solves, const int2* items, int tiles, int rows, int nsolves,
-                                  int nsteps, bool first, bool last, int* err, cudaStream_t s) {
-  return with_buffer(s, [&](ExHead* ex) {
+cudaError_t launch_resident_batch(const BatchSolve* solves, const int2* items, int tiles, int rows, int nsteps,
+                                  bool first, bool last, int* err, cudaStream_t s) {
+  return with_buffer(s, nsteps, [&](ulonglong2* ex, uint32_t tag0) {
     auto k = rows == 4 ? (few<4>(tiles) ? k_resident_batch<4, few_ctas(4)> : k_resident_batch<4, more_ctas(4)>)
                        : (few<8>(tiles) ? k_resident_batch<8, few_ctas(8)> : k_resident_batch<8, more_ctas(8)>);
-    return launch_coop(k, tiles, threads_of(rows), s, solves, items, ex, nsolves, nsteps, (int)first, (int)last, err);
+    return launch_coop(k, tiles, threads_of(rows), s, solves, items, ex, tag0, nsteps, (int)first, (int)last, err);
   });
 }
 

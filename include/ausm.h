@@ -200,6 +200,11 @@ int ausm_time_steps(ausm_solver* h, int n, int reps, float* ms_out);
  * The call waits for the device to be idle, so work queued before it keeps the bound it
  * was queued under.  Restore 65536 afterwards. */
 int ausm_debug_set_wait_polls(unsigned polls);
+/* Test hook: the 32-bit tag with which the next resident launches on the current device mark
+ * the tile edges that they exchange (1 in a new exchange buffer; it goes on by one per RK
+ * stage), so that a test reaches the end of the tags' range.  Make it with no step in
+ * flight, and raise the tag only: a tag that the buffers have seen must not come again. */
+int ausm_debug_set_exchange_tag(unsigned tag);
 /* Tile-height autotuner of the fused engine (no counterpart in the reference): times
  * the TMA stage kernel for tiles of 32 x 8, 32 x 16 and 32 x 32 cells on this solve's
  * grid and state and keeps the fastest for its steps (cached per M, N and scheme for the
