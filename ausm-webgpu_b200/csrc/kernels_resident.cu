@@ -24,8 +24,9 @@
 // stages, an hour and a half of the smallest grids): so whoever uses it next finds none of
 // its own tags in cells that only larger launches write.
 //
-// Every wait is bounded (c_wait_polls); a CTA that gives up sets *err and returns, and
-// the others see *err in their own waits.
+// Every wait is bounded (c_wait_polls); a CTA that gives up sets *err, which the host reads,
+// marks its solve and writes nothing; the other tiles of the solve see the mark in their own
+// waits.  Other solves of a batch, and later launches while *err is set, are not touched.
 //
 // Tiling: the grid is cut into ceil(M / 32) x ceil(N / TY) tiles of nearly equal size,
 // not into full tiles and a remainder: all tiles of a stage take the same time, and no
@@ -127,6 +128,8 @@ template <int TY> struct Smem {
   float4 Qn[TY][TX];          // state at the start of the step
 };
 
+constexpr uint32_t kGaveUp = 1u << 16;  // above the most tiles of a launch
+
 // What a CTA of the launch works on (one tile of one solve).
 struct Job {
   const float4* Qs;
@@ -134,7 +137,8 @@ struct Job {
   const float4* Mi;
   const float4* Mj;
   float* dt;
-  uint32_t* wave;  // [0] max wave speed bits, [1] a launch's accumulator, [2] its finished tiles
+  uint32_t* wave;  // [0] max wave speed bits, [1] a launch's accumulator, [2] its finished tiles, plus kGaveUp
+                   // for each that gave up
   float* out;      // (dt, wave speed) for the host, or null
   int* out_err;    // copy of *err for the host, or null
   int M, N, t;     // t: tile of the solve
@@ -253,6 +257,7 @@ __device__ __forceinline__ void resident_tile(Smem<TY>& sm, const Job& b, const 
     const uint32_t tag = tag0 + st;
     const ulonglong2* e = from + (tag & 1u) * (2 * E::NC);
     const unsigned polls = c_wait_polls * 64u;
+    auto gave_up = [&] { return *(volatile uint32_t*)&b.wave[2] >= kGaveUp; };  // a tile of this solve
     auto arrived = [&](ulonglong2 x, ulonglong2 y) {
       if (tag_of(x.x) != tag || tag_of(x.y) != tag || tag_of(y.x) != tag || tag_of(y.y) != tag) return false;
       *halo = make_float4(value_of(x.x), value_of(x.y), value_of(y.x), value_of(y.y));
@@ -290,7 +295,7 @@ __device__ __forceinline__ void resident_tile(Smem<TY>& sm, const Job& b, const 
             ok = true;
             break;
           }
-          if ((it & 1023u) == 1023u && *(volatile int*)err) break;
+          if ((it & 1023u) == 1023u && gave_up()) break;
           x = ld_pair(e);
           y = ld_pair(e + E::NC);
         }
@@ -303,11 +308,14 @@ __device__ __forceinline__ void resident_tile(Smem<TY>& sm, const Job& b, const 
           ok = true;
           break;
         }
-        if ((it & 1023u) == 1023u && *(volatile int*)err) break;
+        if ((it & 1023u) == 1023u && gave_up()) break;
       }
     }
     if (__syncthreads_or(!ok)) {  // P is complete, or a wait gave up
-      if (tid == 0) atomicExch(err, 1);
+      if (tid == 0) {
+        atomicExch(err, 1);
+        atomicAdd(&b.wave[2], kGaveUp);
+      }
       ok = false;
       break;
     }
@@ -379,25 +387,25 @@ __device__ __forceinline__ void resident_tile(Smem<TY>& sm, const Job& b, const 
     }
   }
   // Every tile of the solve has read wave[0] by the time the last one gets here; that one
-  // publishes the max wave speed of the new state.  Accumulator and count are zero again for
-  // the next launch, also when a wait gave up.
+  // publishes the max wave speed of the new state (none if a tile gave up).  Accumulator and
+  // count are zero again for the next launch, also when a wait gave up.
   if (last) block_max_to(&b.wave[1], wmax);
   if (tid == 0) {
     __threadfence();
-    if (atomicAdd(&b.wave[2], 1u) == (uint32_t)(q.nx * q.ny) - 1) {
+    const uint32_t done = atomicAdd(&b.wave[2], 1u);
+    if ((done & (kGaveUp - 1)) == (uint32_t)(q.nx * q.ny) - 1) {
       __threadfence();
       b.wave[2] = 0u;
       *b.dt = dt;
-      const int e = *(volatile int*)err;
       if (last) {
         const uint32_t bits = atomicExch(&b.wave[1], 0u);
-        if (!e) b.wave[0] = bits;
+        if (done < kGaveUp) b.wave[0] = bits;
         if (b.out) {
           b.out[0] = dt;
           b.out[1] = __uint_as_float(bits);
         }
       }
-      if (b.out_err) *b.out_err = e;
+      if (b.out_err) *b.out_err = *(volatile int*)err;
     }
   }
 }
