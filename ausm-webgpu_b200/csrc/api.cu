@@ -819,8 +819,7 @@ int resident_height(ausm_solver* h, int* rows) {
   return AUSM_OK;
 }
 
-// n fused steps by the resident kernel.  *refused: the device would not take the launch (a
-// process that may use a part of the SMs only), nothing was done.
+// n fused steps by the resident kernel.  *refused (resident_refused): nothing was done.
 int resident_steps(ausm_solver* h, int n, int rows, bool* refused) {
   for (int done = 0; done < n;) {
     const int k = std::min(n - done, kResidentSteps);
@@ -828,8 +827,7 @@ int resident_steps(ausm_solver* h, int n, int rows, bool* refused) {
     const cudaError_t e =
         launch_resident(h->p.scheme, h->Q[h->cur], h->Q[to], h->Mi, h->Mj, h->dt, h->wave, rows, k, done == 0,
                         done + k == n, h->h_dt, (int*)h->h_wave + 2, h->err_flag, h->c, h->M, h->N, h->st);
-    if (done == 0 && e == cudaErrorCooperativeLaunchTooLarge) {
-      cudaGetLastError();
+    if (done == 0 && resident_refused(e)) {
       *refused = true;
       return AUSM_OK;
     }

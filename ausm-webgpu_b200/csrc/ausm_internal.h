@@ -213,6 +213,10 @@ cudaError_t launch_resident(int scheme, const float4* Qs, float4* Qo, const floa
 // Q[cur] to Q[(cur + nsteps) % 3].
 cudaError_t launch_resident_batch(const BatchSolve* solves, const int2* items, int tiles, int rows, int nsteps,
                                   bool first, bool last, int* err, cudaStream_t s);
+// Whether a launch that returned e can be left to the stage kernels (and clears the error):
+// the device would not take it (a process that may use a part of the SMs only), or has no
+// memory for an exchange buffer.
+bool resident_refused(cudaError_t e);
 cudaError_t set_wait_polls_resident(unsigned polls);
 // Test hook: the next tag of every exchange buffer the device has (at least 1).
 void set_exchange_tag(int dev, uint32_t tag);

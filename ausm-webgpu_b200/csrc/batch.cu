@@ -426,8 +426,7 @@ int resident_steps(ausm_batch* b, int n, bool* refused) {
     const cudaError_t e =
         ausm::launch_resident_batch(b->d_solves, b->d_ritems, (int)b->ritems.size(), b->res_rows, k, done == 0,
                                     done + k == n, b->d_err, b->st);
-    if (done == 0 && e == cudaErrorCooperativeLaunchTooLarge) {
-      cudaGetLastError();
+    if (done == 0 && ausm::resident_refused(e)) {
       *refused = true;
       return AUSM_OK;
     }

@@ -501,7 +501,8 @@ int resident_rows(int tiles4, int tiles8) {
 // per solve (a solve would hold up to 72 bytes a cell for it): at most kMaxBuffers per
 // device, created as launches overlap, freed with the device's last solver or batch.  A
 // launch takes the buffer its stream used last, or one whose last launch is over, or waits
-// (on the device) for the oldest.
+// (on the device) for the oldest.  A device without the memory for a first buffer refuses
+// the launch, and the caller steps by the stage kernels, which need none.
 namespace {
 constexpr int kMaxBuffers = 8;
 constexpr size_t kExBytes = 16 * std::max(kMaxTiles4 * Ex<4>::TILE, kMaxTiles8 * Ex<8>::TILE);
@@ -536,14 +537,17 @@ cudaError_t take(Pool& pool, cudaStream_t s, uint32_t stages, Buffer** out) {
     cudaError_t e = cudaMalloc((void**)&b.p, kExBytes);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaMemsetAsync(b.p, 0, kExBytes, s);
-    if (e != cudaSuccess) {
+    if (e == cudaSuccess) {
+      pool.buffers.push_back(b);
+      best = &pool.buffers.back();
+    } else {
       if (b.done) cudaEventDestroy(b.done);
       if (b.p) cudaFree(b.p);
-      return e;
+      if (e != cudaErrorMemoryAllocation || pool.buffers.empty()) return e;
+      cudaGetLastError();  // no memory for one more: share those there are
     }
-    pool.buffers.push_back(b);
-    best = &pool.buffers.back();
-  } else if (!best) {
+  }
+  if (!best) {
     for (Buffer& b : pool.buffers)
       if (!best || b.used < best->used) best = &b;
     const cudaError_t e = cudaStreamWaitEvent(s, best->done, 0);
@@ -633,6 +637,12 @@ cudaError_t launch_resident_batch(const BatchSolve* solves, const int2* items, i
                        : (few<8>(tiles) ? k_resident_batch<8, few_ctas(8)> : k_resident_batch<8, more_ctas(8)>);
     return launch_coop(k, tiles, threads_of(rows), s, solves, items, ex, tag0, nsteps, (int)first, (int)last, err);
   });
+}
+
+bool resident_refused(cudaError_t e) {
+  if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorMemoryAllocation) return false;
+  cudaGetLastError();
+  return true;
 }
 
 cudaError_t set_wait_polls_resident(unsigned polls) { return cudaMemcpyToSymbol(c_wait_polls, &polls, sizeof polls); }
