@@ -223,10 +223,12 @@ void set_exchange_tag(int dev, uint32_t tag);
 // Counts the solvers and batches of a device (+1, -1); with the last one its exchange
 // buffers are freed.
 void resident_user(int dev, int change);
-// Steps of one resident launch at most (10 ms on the largest grids it takes), so that it
-// does not keep the chip from other streams for long; a multiple of 3, so that the buffers
-// rotate as they do step by step.
-constexpr int kResidentSteps = 2049;
+// Steps of one resident launch at most, so that it does not keep the chip from other streams
+// for long: 1.3 ms at 64 x 33, 4.8 ms at 512 x 384 (a step of another solver beside such a
+// launch waits for its end; 2049 steps took 28 ms there).  A launch more costs about 5 us, at
+// 360 steps 0.4 % (512 x 384: 27.36 ms for 2049 steps in one launch, 27.45 in 6, 27.55 in 12).
+// A multiple of 3, so that the buffers rotate as they do step by step.
+constexpr int kResidentSteps = 360;
 
 // ---- full-FP64 engine (kernels_f64.cu, built with -fmad=false) ----
 // The reference-shaped engine in double on its own buffers; vertices are the solver's

@@ -105,12 +105,12 @@ def traffic_from_profile(cells: int):
 
 def launches(engine, M, N, steps):
     """Kernel launches of step(steps): fused, three stage kernels per step (dt is computed in
-    stage 1), or one launch per 2049 steps where the grid's 32 x 8 tiles fit on the chip;
+    stage 1), or one launch per 360 steps where the grid's 32 x 8 tiles fit on the chip;
     reference and F64, two kernels per stage, the dt kernel and the wave-speed reduction."""
     if engine != "fused":
         return 6 * steps + 2
     if -(-M // 32) * -(-N // 8) <= 888 and "AUSM_TILE_ROWS" not in os.environ:
-        return -(-steps // 2049)
+        return -(-steps // 360)
     return 3 * steps
 
 
