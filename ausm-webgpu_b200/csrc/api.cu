@@ -8,6 +8,7 @@
 #include <mutex>
 #include <string>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include "ausm.h"
@@ -395,10 +396,9 @@ int ausm_destroy(ausm_solver* h) {
   if (!h) return AUSM_OK;
   if (h->batch) ausm_batch_remove(h->batch, h);
   cudaSetDevice(h->dev);
-  if (h->counted) resident_user(h->dev, -1);
   if (h->st) cudaStreamSynchronize(h->st);
-  void* dptrs[] = {h->V, h->Vd, h->Mi, h->Mj, h->Q[0], h->Q[1], h->Q[2], h->S[0], h->S[1], h->S[2], h->fx, h->fy, h->res,
-                   h->flen, h->area, h->staging, h->cp, h->wave, h->dt, h->parts, h->move, h->err_flag};
+  if (h->counted) resident_user(h->dev, -1);
+  void* dptrs[] = {h->block, h->S[0], h->S[1], h->S[2], h->fx, h->fy, h->res, h->flen, h->area, h->staging, h->cp};
   for (void* d : dptrs)
     if (d) cudaFree(d);
   delete h->f64;
@@ -444,16 +444,28 @@ int ausm_create(int M, int N, ausm_solver** out) {
   TRY(cudaEventCreate(&h->e0));
   TRY(cudaEventCreate(&h->e1));
   size_t n = (size_t)M * N;
-  TRY(dalloc(&h->V, (size_t)M * (N + 1)));
-  TRY(dalloc(&h->Vd, (size_t)M * (N + 1)));
-  TRY(dalloc(&h->Mi, n));
-  TRY(dalloc(&h->Mj, (size_t)M * (N + 1)));
-  for (auto& q : h->Q) TRY(dalloc(&q, n));
-  TRY(dalloc(&h->wave, 4));
-  TRY(dalloc(&h->dt, 4));
-  TRY(dalloc(&h->parts, 2 * (size_t)kMaxParts));
-  TRY(dalloc(&h->move, 4));
-  TRY(dalloc(&h->err_flag, 1));
+  // one device block, its parts at multiples of 512 bytes
+  size_t bytes = 0;
+  auto part = [&](auto** p, size_t count) {
+    *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(reinterpret_cast<uintptr_t>(h->block) + bytes);
+    bytes += (count * sizeof(**p) + 511) / 512 * 512;
+  };
+  auto lay_out = [&] {
+    bytes = 0;
+    part(&h->V, (size_t)M * (N + 1));
+    part(&h->Vd, (size_t)M * (N + 1));
+    part(&h->Mi, n);
+    part(&h->Mj, (size_t)M * (N + 1));
+    for (auto& q : h->Q) part(&q, n);
+    part(&h->wave, 4);
+    part(&h->dt, 4);
+    part(&h->parts, 2 * (size_t)kMaxParts);
+    part(&h->move, 4);
+    part(&h->err_flag, 1);
+  };
+  lay_out();  // its size
+  TRY(dalloc(&h->block, bytes));
+  lay_out();
   TRY(cudaMemsetAsync(h->err_flag, 0, sizeof(int), h->st));
   TRY(cudaMallocHost((void**)&h->h_dt, 4 * sizeof(float)));
   TRY(cudaMallocHost((void**)&h->h_wave, 4 * sizeof(uint32_t)));
@@ -467,6 +479,8 @@ int ausm_create(int M, int N, ausm_solver** out) {
   }
   resident_user(h->dev, 1);
   h->counted = true;
+  if (const int rows = resident_rows(resident_tiles(M, N, 4), resident_tiles(M, N, 8)))
+    resident_reserve(h->dev, resident_tiles(M, N, rows), rows, h->st);
   ausm_default_params(&h->p);
   h->speed_now = inflow_target(h->p);
   make_consts(h);

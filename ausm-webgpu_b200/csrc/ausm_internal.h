@@ -220,9 +220,12 @@ bool resident_refused(cudaError_t e);
 cudaError_t set_wait_polls_resident(unsigned polls);
 // Test hook: the next tag of every exchange buffer the device has (at least 1).
 void set_exchange_tag(int dev, uint32_t tag);
-// Counts the solvers and batches of a device (+1, -1); with the last one its exchange
-// buffers are freed.
+// Counts the solvers, batches and servers of a device (+1, -1); with the last one its
+// exchange buffers are freed.
 void resident_user(int dev, int change);
+// Sees to it that the device (the current one) has an exchange buffer for a launch of that
+// many tiles; a new one is cleared on s.
+void resident_reserve(int dev, int tiles, int rows, cudaStream_t s);
 // Steps of one resident launch at most, so that it does not keep the chip from other streams
 // for long: 1.3 ms at 64 x 33, 4.8 ms at 512 x 384 (a step of another solver beside such a
 // launch waits for its end; 2049 steps took 28 ms there).  A launch more costs about 5 us, at

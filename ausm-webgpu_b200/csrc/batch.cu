@@ -549,7 +549,9 @@ int ausm_batch_add(ausm_batch* b, ausm_solver* h) {
   h->batch = b;
   h->st = b->st;
   relayout(b);
-  return ensure_capacity(b);
+  if ((rc = ensure_capacity(b))) return rc;
+  if (b->res_rows) ausm::resident_reserve(b->dev, (int)b->ritems.size(), b->res_rows, b->st);
+  return AUSM_OK;
 }
 
 int ausm_batch_remove(ausm_batch* b, ausm_solver* h) {

@@ -499,15 +499,22 @@ int resident_rows(int tiles4, int tiles8) {
 // ---- exchange buffers ----
 // A launch needs one for its own duration only, so they are kept for the process and not
 // per solve (a solve would hold up to 72 bytes a cell for it): at most kMaxBuffers per
-// device, created as launches overlap, freed with the device's last solver or batch.  A
-// launch takes the buffer its stream used last, or one whose last launch is over, or waits
-// (on the device) for the oldest.  A device without the memory for a first buffer refuses
+// device, created with a solver or a batch for which none is large enough, so that its steps
+// allocate nothing, and as launches overlap; freed with the device's last solver, batch or
+// server.  A launch takes, of those that are large enough, the buffer its stream used last,
+// or one whose last launch is over, or waits (on the device) for the oldest.  A device without the memory for a first buffer refuses
 // the launch, and the caller steps by the stage kernels, which need none.
 namespace {
 constexpr int kMaxBuffers = 8;
-constexpr size_t kExBytes = 16 * std::max(kMaxTiles4 * Ex<4>::TILE, kMaxTiles8 * Ex<8>::TILE);
+// Up to 9.1 MB, 10 MiB with the rounding.  Sizes up to 1 MiB share mappings with other small arrays (1 us to allocate
+// instead of 340), larger ones take whole mappings of 2 MiB.
+size_t bytes_of(int tiles, int rows) {
+  const size_t need = 16 * tiles * (rows == 4 ? Ex<4>::TILE : Ex<8>::TILE), unit = need <= (1u << 20) ? 1u << 18 : 1u << 21;
+  return (need + unit - 1) / unit * unit;
+}
 struct Buffer {
   ulonglong2* p = nullptr;
+  size_t bytes = 0;
   uint32_t tag = 1;  // of the next launch's first exchange; 0 is that of a cleared buffer
   cudaEvent_t done = nullptr;
   cudaStream_t stream = nullptr;
@@ -521,42 +528,70 @@ struct Pool {
 std::mutex g_pool_mu;
 std::map<int, Pool> g_pool;  // per device
 
-// A buffer for a launch of `stages` stages on s.  With g_pool_mu held and the device current.
-cudaError_t take(Pool& pool, cudaStream_t s, uint32_t stages, Buffer** out) {
-  Buffer* best = nullptr;
+void free_buffer(Buffer& b) {
+  cudaEventSynchronize(b.done);
+  cudaFree(b.p);
+  cudaEventDestroy(b.done);
+}
+
+// One more buffer, cleared on s.  With g_pool_mu held and the device current.
+cudaError_t add_buffer(Pool& pool, size_t bytes, cudaStream_t s) {
+  Buffer b;
+  b.bytes = bytes;
+  cudaError_t e = cudaMalloc((void**)&b.p, bytes);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaMemsetAsync(b.p, 0, bytes, s);
+  if (e == cudaSuccess) e = cudaEventRecord(b.done, s);
+  if (e != cudaSuccess) {
+    if (b.done) cudaEventDestroy(b.done);
+    if (b.p) cudaFree(b.p);
+    return e;
+  }
+  b.stream = s;
+  pool.buffers.push_back(b);
+  return cudaSuccess;
+}
+
+// A buffer of at least `bytes` for a launch of `stages` stages on s.  With g_pool_mu held and
+// the device current.
+cudaError_t take(Pool& pool, cudaStream_t s, size_t bytes, uint32_t stages, Buffer** out) {
+  Buffer *best = nullptr, *oldest = nullptr;  // oldest: of those large enough
   for (Buffer& b : pool.buffers)
-    if (b.stream == s) best = &b;
+    if (b.bytes >= bytes) {
+      if (b.stream == s) best = &b;
+      if (!oldest || b.used < oldest->used) oldest = &b;
+    }
   if (!best)
     for (Buffer& b : pool.buffers) {
       if (best) break;
+      if (b.bytes < bytes) continue;
       if (cudaEventQuery(b.done) == cudaSuccess) best = &b;
       else cudaGetLastError();  // busy, or not to be asked now: not an error of this thread's calls
     }
-  if (!best && (int)pool.buffers.size() < kMaxBuffers) {
-    Buffer b;
-    cudaError_t e = cudaMalloc((void**)&b.p, kExBytes);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaMemsetAsync(b.p, 0, kExBytes, s);
+  if (!best && ((int)pool.buffers.size() < kMaxBuffers || !oldest)) {
+    if ((int)pool.buffers.size() == kMaxBuffers) {  // all too small: the one unused for longest makes room
+      auto b = std::min_element(pool.buffers.begin(), pool.buffers.end(),
+                                [](const Buffer& x, const Buffer& y) { return x.used < y.used; });
+      free_buffer(*b);
+      pool.buffers.erase(b);
+    }
+    const cudaError_t e = add_buffer(pool, bytes, s);
     if (e == cudaSuccess) {
-      pool.buffers.push_back(b);
       best = &pool.buffers.back();
     } else {
-      if (b.done) cudaEventDestroy(b.done);
-      if (b.p) cudaFree(b.p);
-      if (e != cudaErrorMemoryAllocation || pool.buffers.empty()) return e;
+      if (e != cudaErrorMemoryAllocation || !oldest) return e;
       cudaGetLastError();  // no memory for one more: share those there are
     }
   }
   if (!best) {
-    for (Buffer& b : pool.buffers)
-      if (!best || b.used < best->used) best = &b;
+    best = oldest;
     const cudaError_t e = cudaStreamWaitEvent(s, best->done, 0);
     if (e != cudaSuccess) return e;
   }
   best->stream = s;
   best->used = ++pool.clock;
   if (best->tag > UINT32_MAX - stages) {  // the tags would wrap: start again on a cleared buffer
-    const cudaError_t e = cudaMemsetAsync(best->p, 0, kExBytes, s);
+    const cudaError_t e = cudaMemsetAsync(best->p, 0, best->bytes, s);
     if (e != cudaSuccess) return e;
     best->tag = 1;
   }
@@ -578,10 +613,10 @@ cudaError_t launch_coop(void (*kern)(KArgs...), int ctas, int threads, cudaStrea
   return cudaLaunchKernelEx(&cfg, kern, static_cast<Args&&>(args)...);
 }
 
-// Takes a buffer of the current device for `nsteps` steps on s, calls launch(cells, first
-// tag), notes when the buffer is free.  None of it belongs to a stream capture another
+// Takes a buffer of the current device for `nsteps` steps of `tiles` tiles on s, calls
+// launch(cells, first tag), notes when the buffer is free.  None of it belongs to a stream capture another
 // thread may have open.
-template <class F> cudaError_t with_buffer(cudaStream_t s, int nsteps, F launch) {
+template <class F> cudaError_t with_buffer(cudaStream_t s, int tiles, int rows, int nsteps, F launch) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
@@ -590,7 +625,7 @@ template <class F> cudaError_t with_buffer(cudaStream_t s, int nsteps, F launch)
   {
     std::lock_guard<std::mutex> lk(g_pool_mu);
     Buffer* b = nullptr;
-    e = take(g_pool[dev], s, 3u * nsteps, &b);
+    e = take(g_pool[dev], s, bytes_of(tiles, rows), 3u * nsteps, &b);
     if (e == cudaSuccess) {
       e = launch(b->p, b->tag);
       if (e == cudaSuccess) b->tag += 3u * nsteps;
@@ -613,18 +648,25 @@ void resident_user(int dev, int change) {
   Pool& pool = g_pool[dev];
   pool.users += change;
   if (pool.users > 0) return;
-  for (Buffer& b : pool.buffers) {  // cudaFree waits for the device
-    cudaFree(b.p);
-    cudaEventDestroy(b.done);
-  }
+  for (Buffer& b : pool.buffers) free_buffer(b);
   pool.buffers.clear();
+}
+
+void resident_reserve(int dev, int tiles, int rows, cudaStream_t s) {
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  Pool& pool = g_pool[dev];
+  const size_t bytes = bytes_of(tiles, rows);
+  if ((int)pool.buffers.size() == kMaxBuffers) return;
+  for (const Buffer& b : pool.buffers)
+    if (b.bytes >= bytes) return;
+  if (add_buffer(pool, bytes, s) != cudaSuccess) cudaGetLastError();  // a step will ask again
 }
 
 cudaError_t launch_resident(int scheme, const float4* Qs, float4* Qo, const float4* Mi, const float4* Mj, float* dt,
                             uint32_t* wave, int rows, int nsteps, bool first, bool last, float* out, int* out_err,
                             int* err, const Consts& c, int M, int N, cudaStream_t s) {
   const int sf = scheme + (c.muscl > 0 ? 4 : 0), tiles = resident_tiles(M, N, rows);
-  return with_buffer(s, nsteps, [&](ulonglong2* ex, uint32_t tag0) {
+  return with_buffer(s, tiles, rows, nsteps, [&](ulonglong2* ex, uint32_t tag0) {
     return launch_coop(rows == 4 ? kernel_of<4>(sf, tiles) : kernel_of<8>(sf, tiles), tiles, threads_of(rows), s, Qs,
                        Qo, Mi, Mj, dt, wave, ex, tag0, nsteps, (int)first, (int)last, out, out_err, err, c, M, N);
   });
@@ -632,7 +674,7 @@ cudaError_t launch_resident(int scheme, const float4* Qs, float4* Qo, const floa
 
 cudaError_t launch_resident_batch(const BatchSolve* solves, const int2* items, int tiles, int rows, int nsteps,
                                   bool first, bool last, int* err, cudaStream_t s) {
-  return with_buffer(s, nsteps, [&](ulonglong2* ex, uint32_t tag0) {
+  return with_buffer(s, tiles, rows, nsteps, [&](ulonglong2* ex, uint32_t tag0) {
     auto k = rows == 4 ? (few<4>(tiles) ? k_resident_batch<4, few_ctas(4)> : k_resident_batch<4, more_ctas(4)>)
                        : (few<8>(tiles) ? k_resident_batch<8, few_ctas(8)> : k_resident_batch<8, more_ctas(8)>);
     return launch_coop(k, tiles, threads_of(rows), s, solves, items, ex, tag0, nsteps, (int)first, (int)last, err);

@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "ausm.h"
+#include "ausm_internal.h"
 #include "solver_internal.h"
 
 namespace {
@@ -111,6 +112,7 @@ struct ausm_server {
   double budget = 0.0;
   int max_active = 1, chunk = 100, flags = 0;
   int dev = -1;
+  bool counted = false;  // a user of the device's exchange buffers, which stay between its requests
   std::mutex mu;       // everything below except the CUDA objects
   std::mutex pump_mu;  // one round at a time
   std::condition_variable cv;
@@ -290,6 +292,10 @@ int pump_round(ausm_server* s, int* remaining) {
     }
   } else {
     cudaSetDevice(s->dev);
+  }
+  if (!s->counted) {
+    ausm::resident_user(s->dev, 1);
+    s->counted = true;
   }
   if (!(s->flags & AUSM_SERVE_PLAIN) && !s->batch) {
     int rc = ausm_batch_create(&s->batch);
@@ -479,6 +485,7 @@ int ausm_server_destroy(ausm_server* s) {
       q->h = nullptr;
     }
   if (s->batch) ausm_batch_destroy(s->batch);
+  if (s->counted) ausm::resident_user(s->dev, -1);
   delete s;
   return AUSM_OK;
 }

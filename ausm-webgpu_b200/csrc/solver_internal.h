@@ -21,6 +21,8 @@ struct ausm_solver {
   std::vector<double> body, outer;  // M x 2
   bool has_body = false, has_outer = false, has_grid = false, has_state = false;
   double stretch = 0.0;
+  char* block = nullptr;  // the device memory of the arrays from V to Q and of wave, dt, parts, move and err_flag:
+                          // a new mapping and its release cost 0.6 ms each
   float2* V = nullptr;    // vertices, FP32 (reference layout, API, reference engine)
   double2* Vd = nullptr;  // vertices, FP64 (multicolor generator, metrics, forces)
   float4* Mi = nullptr;   // FP64-computed face records, i-faces [N][M]

@@ -45,48 +45,81 @@ for p in ({root!r}, {root!r} + "/tests", {root!r} + "/ausm-webgpu_b200"):
 from ausm import Batch
 from test_gpu_edges import solver
 
-def members():
-    return [solver(96, 40), solver(65, 33, scheme="AUSM+-up")]
-
-def steps(s, sols, b):
-    return [s.step(3), b.step(2), s.step(1), b.step(3), s.state()] + [x.state() for x in sols]
+def steps(s):
+    out = [s.step(3), s.step(1)]
+    with Batch(graphs=False) as b:
+        b.add(s)
+        out += [b.step(2), b.step(3)]
+    return out + [s.state()]
 
 os.environ["AUSM_TILE_ROWS"] = "16"  # the stage kernels, loaded before the memory is taken
-s, sols, b = solver(128, 96), members(), Batch(graphs=False)
-for x in sols:
-    b.add(x)
-want = steps(s, sols, b)
-b.close()
-for x in [s] + sols:
-    x.close()
+with solver(300, 200) as s:
+    want = steps(s)
 del os.environ["AUSM_TILE_ROWS"]
 os.environ["AUSM_AUTOTUNE"] = "0"
 
 cu = C.CDLL("libcuda.so.1")
 held = []
-def fill(size):
-    p = C.c_void_p()
-    while cu.cuMemAlloc_v2(C.byref(p), C.c_size_t(size)) == 0:
-        held.append(p)
-        p = C.c_void_p()
 
-def give_back(n):
-    for _ in range(n):
-        assert cu.cuMemFree_v2(held.pop()) == 0
+def take(size):
+    p = C.c_void_p()
+    if cu.cuMemAlloc_v2(C.byref(p), C.c_size_t(size)):
+        return False
+    held.append(p)
+    return True
+
+def give_back(p):
+    held.remove(p)
+    assert cu.cuMemFree_v2(p) == 0
 
 for k in range(34, 20, -1):
-    fill(1 << k)
-give_back(1)
-fill(2 << 20)
-give_back(3)
-fill(8 << 20)  # the rest holds small solvers, but no exchange buffer (9.1 MB)
-s, sols, b = solver(128, 96), members(), Batch(graphs=False)
-for x in sols:
-    b.add(x)
-got = steps(s, sols, b)
-give_back(len(held))
+    while take(1 << k):
+        pass
+while not take(8 << 20):  # the solver's arrays (6.3 MB)
+    give_back(held[-1])
+mine = held[-1]
+while take(2 << 20):
+    pass
+for p in [mine] + [p for p in held if p is not mine][-2:]:  # and 4 MiB: less than its exchange buffer
+    give_back(p)
+s = solver(300, 200)
+got = steps(s)
+while held:
+    give_back(held[-1])
 for x, y in zip(got, want):
     np.testing.assert_array_equal(x, y)
+'''
+
+KEEP = r'''
+import ctypes as C, sys
+for p in ({root!r}, {root!r} + "/tests", {root!r} + "/ausm-webgpu_b200"):
+    sys.path.insert(0, p)
+import ausm
+from test_gpu_edges import solver
+
+cu = C.CDLL("libcuda.so.1")
+
+def free():
+    a, b = C.c_size_t(), C.c_size_t()
+    assert cu.cuMemGetInfo_v2(C.byref(a), C.byref(b)) == 0
+    return a.value
+
+for k in range(3):  # the first turn loads the kernels
+    with solver(300, 200) as s:
+        s.synchronize()
+        before = free()
+        s.step(2)
+        assert k == 0 or free() == before, "a step allocated or freed device memory"
+s = solver(300, 200)
+s.close()
+none = free()
+with ausm.Server(1e9, chunk_steps=10, plain=True) as srv:
+    for k in range(2):
+        srv.submit(ausm.make_request(300, 200, naca4=12, mach=0.5, far_radius=10.0, grid_iters=20, max_steps=20))
+        srv.drain()
+        held = none - free()
+        assert held > 4e6, f"{{held}} bytes held between requests"
+assert free() == none, "the buffer was not given back"
 '''
 
 
@@ -102,6 +135,13 @@ def test_tags_start_again_on_a_cleared_buffer():
     """One buffer, first tag 1.  Past the range's end the next launch would read the first
     one's edges as its neighbours' had the buffer not been cleared."""
     run(WRAP)
+
+
+def test_buffer_is_kept_and_given_back():
+    """One solver at a time: the buffer comes with its creation, so that a step allocates
+    nothing.  A server keeps it between its requests, also one that serves them singly, and
+    gives it back at its end."""
+    run(KEEP)
 
 
 def test_steps_without_memory_for_a_buffer():
