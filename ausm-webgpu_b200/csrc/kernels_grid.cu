@@ -298,14 +298,18 @@ void sweeps_d(const double2* src, double2* dst, const double2* ends, int M, int 
   allow_smem<kern>((MAX_H + 2 * NC * S) * ROW);
   launch_pdl(kern, g, dim3(32 * NW), (size_t)(h + 2 * NC * S) * ROW, s, src, dst, ends, M, N, sweeps, omega, move);
 }
-// Two sweeps to a launch while the tiles of that halo (48 or 40 columns, up to 32 rows) fit
-// the SMs one each: there a launch is bound by its fixed cost and the latency of the colour
-// steps (us per sweep, one sweep / two: 128 x 96 3.6 / 3.0, 257 x 131 5.2 / 4.7, 512 x 384
-// 6.3 / 5.4; four: 3.5 and more).  Beyond, the wider tiles of one sweep (56 or 52 columns)
-// win: 1024 x 768 13.4 / 14.1 (before the loads were batched).
+// One or two sweeps to a launch.  Two halve the launches and the trips through L2, for a
+// deeper halo (tiles of 48 columns instead of 56, with odd M 40 instead of 52).
+// Even M: two while the tiles of one sweep are cut for two rounds of the SMs at most; three
+// rounds are lower tiles that run three to an SM, and one sweep wins (us per sweep, one /
+// two: 64 x 33 3.0 / 2.7, 512 x 384 6.6 / 5.3, 640 x 480 8.2 / 7.0, 900 x 600 13.1 / 11.4,
+// 4096 x 160 14.1 / 12.6; beyond, 1000 x 650 11.1 / 12.7, 256 x 2400 11.0 / 13.7, 1024 x 768
+// 13.0 / 15.4).  Odd M, whose halos are half as deep again: two while their tiles fit the SMs
+// one each (129 x 97 4.3 / 4.3, 201 x 151 4.5 / 4.7, 401 x 300 6.9 / 6.5, 513 x 300 7.5 / 7.1;
+// beyond, 513 x 385 8.6 / 8.7, 721 x 481 11.7 / 11.3, 801 x 600 15.0 / 16.8).
 bool two_sweeps(int M, int N) {
-  const int ti = GW - 2 * 2 * ((M & 1) ? 6 : 4);
-  return (long long)((M + ti - 1) / ti) * ((N - 1 + 31) / 32) <= kSMs;
+  auto tiles = [&](int cols, int rows) { return (long long)((M + cols - 1) / cols) * ((N - 1 + rows - 1) / rows); };
+  return M & 1 ? tiles(40, 32) <= kSMs : tiles(56, 40) <= 2 * kSMs;
 }
 }  // namespace
 
