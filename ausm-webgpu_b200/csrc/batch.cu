@@ -253,19 +253,26 @@ void relayout(ausm_batch* b) {
   b->uploaded = false;
 }
 
-// Brings the device descriptors up to date with the members' host state.
-int sync_descriptors(ausm_batch* b) {
+// Brings the device descriptors up to date with the members' host state.  A stream capture
+// cannot hold that: its replays would read the host's tables, which by then are others or
+// gone, so a captured step whose batch has changed since its last direct call is refused.
+int sync_descriptors(ausm_batch* b, bool captured = false) {
+  auto refuse = [&] {
+    return bfail(b, AUSM_ERR_STATE, "the batch has changed: take a step of it before one is captured");
+  };
   for (size_t k = 0; k < b->members.size(); k++)
     if (group_key(b->members[b->order[k]]) != b->mirror[k].scheme) {  // regroup
       relayout(b);
       break;
     }
+  if (captured && !b->uploaded) return refuse();
   if (int rc = ensure_capacity(b)) return rc;  // fewer members may have more (resident) work items
   bool changed = !b->uploaded;
   for (size_t k = 0; k < b->members.size(); k++) {
     BatchSolve d = describe(b->members[b->order[k]], b->mirror[k].tile0, b->mirror[k].chunk0, b->mirror[k].rtile0,
                             maps_of(b, (int)k));
     if (std::memcmp(&d, &b->mirror[k], sizeof d) != 0) {
+      if (captured) return refuse();
       b->mirror[k] = d;
       changed = true;
     }
@@ -605,7 +612,7 @@ int batch_step_impl(ausm_batch* b, int n, float* dt_wave, bool read_err) {
     if (resident) b->res_stepped = true;
   }
   if (!resident) {
-    if ((rc = tune_rows(b, captured)) || (rc = sync_descriptors(b)) || (rc = run_steps(b, n))) return rc;
+    if ((rc = tune_rows(b, captured)) || (rc = sync_descriptors(b, captured)) || (rc = run_steps(b, n))) return rc;
   }
   for (size_t k = 0; k < b->members.size(); k++) {
     ausm_solver* h = b->members[b->order[k]];

@@ -38,6 +38,17 @@ class Graph:
         self.ok(self.cu.cuGraphExecDestroy(self.exec))
 
 
+def refused(stream, fn, code):
+    """fn must fail with `code` inside a capture, and leave the capture itself valid."""
+    from ausm import AusmError
+
+    def go():
+        with pytest.raises(AusmError) as e:
+            fn()
+        assert e.value.code == code
+    Graph(stream, go).close()
+
+
 def stream_of(s):
     from ausm import _lib
     st = C.c_void_p()
@@ -88,4 +99,35 @@ def test_captured_batch_step_beside_direct_steps():
     for x, y in zip(mine + [other], twins + [other_twin]):
         np.testing.assert_array_equal(x.state(), y.state())
     for s in mine + twins + [other, other_twin]:
+        s.close()
+
+
+def test_captured_batch_step_refuses_to_upload(monkeypatch):
+    """A captured step cannot bring the device's tables up to date (a replay would read host
+    memory that has changed or gone): before the first direct call, after a parameter change
+    and after a membership change it is refused, and a direct step makes it possible again."""
+    from ausm import Batch, _lib
+    monkeypatch.setenv("AUSM_TILE_ROWS", "8")  # a fixed height: nothing to tune
+    sols = [solver(M, N, scheme=sc) for M, N, sc in SIZES]
+    st = None
+    with Batch(graphs=False) as b:
+        def no():
+            refused(st, lambda: b.step(3, wait=False), _lib.ERR_STATE)
+        for s in sols:
+            b.add(s)
+        st = stream_of(sols[0])
+        no()
+        b.step(3)
+        sols[0].set_params(mach=0.7)
+        no()
+        b.step(3)
+        b.remove(sols[1])
+        no()
+        b.step(3)
+        g = Graph(st, lambda: b.step(3, wait=False))
+        g.launch()
+        out = b.step(1)
+        g.close()
+    assert np.all(np.isfinite(out))
+    for s in sols:
         s.close()
