@@ -96,7 +96,7 @@ int forced_tile_rows() {
   return r == 8 || r == 16 || r == 32 ? r : 0;
 }
 
-int tuned_tile_rows(ausm_solver* h, bool force, int* rows) {
+int tuned_tile_rows(ausm_solver* h, bool force, bool may_measure, int* rows) {
   *rows = 16;
   if (!h->tma[1].ok) return AUSM_OK;  // per-thread kernels: 16 rows
   if (const int r = forced_tile_rows())
@@ -110,9 +110,6 @@ int tuned_tile_rows(ausm_solver* h, bool force, int* rows) {
     *rows = h->tile_rows;
     return AUSM_OK;
   }
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(h->st, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone)
-    return AUSM_OK;  // a grid whose steps have all been resident so far: not tuned yet
   const auto key = std::make_tuple(h->M, h->N, h->p.scheme);
   if (!force) {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -121,6 +118,13 @@ int tuned_tile_rows(ausm_solver* h, bool force, int* rows) {
       *rows = h->tile_rows = it->second;
       return AUSM_OK;
     }
+  }
+  if (!may_measure) return AUSM_OK;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(h->st, &cap) == cudaSuccess && cap != cudaStreamCaptureStatusNone) {
+    h->err = "tile autotuning times and waits, which a stream capture does not allow: tune before it";
+    set_thread_error(h->err);
+    return AUSM_ERR_CUDA;
   }
   const int a = h->cur, b = (a + 1) % 3;
   const double cells = (double)h->M * h->N;
@@ -822,14 +826,17 @@ int read_dt(ausm_solver* h, float* dt_out) {
 
 // Tile height of the resident kernel for h's next steps, 0: the stage kernels.  A stream
 // capture stays on those: a captured launch would hold an exchange buffer that others use.
-int resident_height(ausm_solver* h, int* rows) {
+// *captured: it is only for that (direct steps of h are resident).
+int resident_height(ausm_solver* h, int* rows, bool* captured) {
   *rows = 0;
+  *captured = false;
   if (forced_tile_rows()) return AUSM_OK;
   const int r = resident_rows(resident_tiles(h->M, h->N, 4), resident_tiles(h->M, h->N, 8));
   if (!r) return AUSM_OK;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   CU(h, cudaStreamIsCapturing(h->st, &cap));
-  if (cap == cudaStreamCaptureStatusNone) *rows = r;
+  *captured = cap != cudaStreamCaptureStatusNone;
+  if (!*captured) *rows = r;
   return AUSM_OK;
 }
 
@@ -877,8 +884,8 @@ int step_impl(ausm_solver* h, int n, float* dt_out, bool read_err) {
     return AUSM_OK;
   }
   int res_rows = 0;
-  if (h->engine == AUSM_ENGINE_FUSED && n > 0 && (rc = resident_height(h, &res_rows))) return rc;
-  bool refused = false;
+  bool captured = false, refused = false;
+  if (h->engine == AUSM_ENGINE_FUSED && n > 0 && (rc = resident_height(h, &res_rows, &captured))) return rc;
   if (res_rows && (rc = resident_steps(h, n, res_rows, &refused))) return rc;
   if (res_rows && !refused) {
     ramp_after_steps(h, n);
@@ -892,7 +899,8 @@ int step_impl(ausm_solver* h, int n, float* dt_out, bool read_err) {
     if (h->engine != AUSM_ENGINE_FUSED) CU(h, cudaMemsetAsync(h->wave, 0, sizeof(uint32_t), s));
     if (h->engine == AUSM_ENGINE_FUSED) {
       int rows = 16;
-      if ((rc = tuned_tile_rows(h, false, &rows))) return rc;
+      // direct steps that are resident tune nothing, and a capture cannot
+      if ((rc = tuned_tile_rows(h, false, !captured, &rows))) return rc;
       for (int k = 0; k < n; k++) {
         int a = h->cur, b = (a + 1) % 3, c3 = (a + 2) % 3;
         TmaMapsLaunch t1, t2, t3;
@@ -1087,7 +1095,7 @@ int ausm_autotune(ausm_solver* h, int force, int* rows) {
   int r = 16;
   if (h->engine == AUSM_ENGINE_FUSED) {
     launch_dt(h->wave, h->dt, h->c.maxdt, h->c.cfl, h->st);
-    if ((rc = tuned_tile_rows(h, force != 0, &r))) return rc;
+    if ((rc = tuned_tile_rows(h, force != 0, true, &r))) return rc;
   }
   if (rows) *rows = r;
   return AUSM_OK;

@@ -364,6 +364,7 @@ int tune_rows(ausm_batch* b, bool captured) {
   }
   if (b->tuned_rows && cells <= 2.0 * b->tuned_cells && 2.0 * cells >= b->tuned_cells) return AUSM_OK;
   if (captured && b->res_rows && b->res_stepped) return AUSM_OK;
+  BNEED(b, !captured, AUSM_ERR_CUDA, "tuning times and waits, which a stream capture does not allow: step before it");
   const int reps = (int)std::max(5.0, std::min(100.0, 1.0e8 / std::max(cells, 1.0)));
   float best_ms[3] = {INFINITY, INFINITY, INFINITY};
   const int cand[3] = {8, 16, 32};

@@ -62,6 +62,7 @@ void set_thread_error(const std::string& msg);
 // The tile height AUSM_TILE_ROWS fixes for the stage kernels (8, 16 or 32), or 0.  A fixed
 // height also keeps small grids on the stage kernels.
 int forced_tile_rows();
-int tuned_tile_rows(ausm_solver* h, bool force, int* rows);
+// may_measure false: 16 rows where a tuning run would be needed.
+int tuned_tile_rows(ausm_solver* h, bool force, bool may_measure, int* rows);
 inline int tile_index(int rows) { return rows == 8 ? 0 : (rows == 32 ? 2 : 1); }
 }  // namespace ausm

@@ -131,3 +131,21 @@ def test_captured_batch_step_refuses_to_upload(monkeypatch):
     assert np.all(np.isfinite(out))
     for s in sols:
         s.close()
+
+
+def test_captured_tuning_is_refused():
+    """Tuning times and waits, which a capture does not allow: a captured step of a grid too
+    large to be resident needs its tile height tuned before, and so does ausm_autotune itself
+    at any size; a batch needs a step before.  Neither capture nor solver is the worse for the
+    attempt."""
+    from ausm import Batch, _lib
+    for M, N, call in ((1030, 411, lambda s: s.step(3, wait=False)), (71, 37, lambda s: s.autotune())):
+        s = solver(M, N)
+        refused(stream_of(s), lambda: call(s), _lib.ERR_CUDA)
+        assert s.autotune() in (8, 16, 32)
+        assert np.isfinite(s.step(2))
+        with Batch(graphs=False) as b:
+            b.add(s)
+            refused(stream_of(s), lambda: b.step(3, wait=False), _lib.ERR_CUDA)
+            assert np.all(np.isfinite(b.step(2)))
+        s.close()
