@@ -41,7 +41,8 @@ def device_count() -> int:
 
 def set_wait_polls(polls: int):
     """Test hook: polls (0..65536, the default) of the stage kernels' first bounded wait
-    for each TMA box on the current device; 0 makes every such wait give up at once."""
+    for each TMA box, and 64 times as many of the resident kernel's wait for an edge, on the
+    current device; 0 makes every such wait give up at once."""
     check(lib().ausm_debug_set_wait_polls(int(polls)))
 
 
@@ -217,7 +218,8 @@ class Solver:
 
     def autotune(self, force: bool = False) -> int:
         """Tile height (8, 16 or 32 rows) of the fused stage kernel for this solve, measured
-        on first use (or again with force); returns the height in use."""
+        on first use (or again with force); returns the height in use.  Grids up to 227 K
+        cells step by the resident kernel and need it for stream captures alone."""
         r = C.c_int()
         self._c(lib().ausm_autotune(self.h, int(bool(force)), C.byref(r)))
         return r.value
@@ -230,11 +232,12 @@ class Solver:
 
 
 class Batch:
-    """Many solves stepped together: one kernel launch per RK stage and scheme over the
-    tiles of every member (no counterpart in the reference, which steps one grid).
+    """Many solves stepped together (no counterpart in the reference, which steps one grid):
+    in one launch while the tiles of all members fit on the chip together, else by one kernel
+    launch per RK stage and scheme, the n-step sequence replayed from a CUDA graph.
 
     Members keep their own dt, scheme and parameters; a member's results are the same
-    alone or in any batch.  The n-step sequence is replayed from a CUDA graph."""
+    alone or in any batch."""
 
     def __init__(self, graphs: bool = True):
         b = C.c_void_p()

@@ -1,6 +1,8 @@
 // ausm_batch_*: many independent solves advanced by one kernel launch per RK stage and
 // scheme group (kernels_batch.cu), the n-step sequence captured as a CUDA graph in which
 // the scheme groups are independent branches (their stage chains overlap on the GPU).
+// Members whose tiles all fit on the chip together take their steps in one resident launch
+// instead (kernels_resident.cu), without graph or tuning.
 //
 // Device data: one BatchSolve descriptor per member (its buffers, constants, scheme,
 // first work item and current-buffer index), the members' tensor maps (kBatchMaps

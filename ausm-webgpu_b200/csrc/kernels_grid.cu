@@ -8,7 +8,7 @@
 // tiles that own them, from the same operands, so the result has the bits of one launch
 // per colour or sweep.  One launch per colour left three lanes of four idle, read the
 // nine neighbours from L2 with a stride and cost a launch per colour.  Measured on B200,
-// FP64 multicolour, us per sweep before / now: 128 x 96 18.4 / 3.0, 512 x 384 25.1 / 5.5,
+// FP64 multicolour, us per sweep before / now: 128 x 96 18.4 / 2.9, 512 x 384 25.1 / 5.4,
 // 1024 x 768 41.6 / 13.0, 4096 x 3072 563 / 168.  What is left at 1024 x 768: some 5 us of FP64
 // arithmetic (72 operations a vertex at half rate, halo and idle lanes included) and the
 // tiles' way in and out of L2, which all CTAs of the launch take at the same time; on

@@ -15,7 +15,7 @@
 // Bound by its IEEE divisions and square roots (some 50 a cell and stage) and by latency.  A
 // step of 510 x 381 (AUSM+-up) took 100 us with one kernel per dispatch (full copies in the
 // boundary pass, the residual through memory, eight conversions to primitives per cell),
-// 75 us with those kernels under programmatic dependent launch, and takes 52 us.
+// 75 us with those kernels under programmatic dependent launch, and takes 53 us.
 #include "ausm_internal.h"
 #include "tma.cuh"
 

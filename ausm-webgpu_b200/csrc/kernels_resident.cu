@@ -10,7 +10,7 @@
 //
 // Why: on these grids the stage kernels (kernels_fused.cu) are bound by latency, not by
 // work.  Each launch drains the chip, fetches records and state again and waits for the
-// last CTA of the grid; a stage of 128 x 96 cells took 5 us and one of 512 x 384 7.2 us
+// last CTA of the grid; a stage of 128 x 96 cells takes 4.1 us and one of 512 x 384 7.0 us
 // with about 1.6 us of arithmetic in it.
 //
 // Exchange: every 8-byte word carries one float and a 32-bit tag (the number of the stage
@@ -40,18 +40,21 @@
 // interleaved, the fifth takes the top row and the right column; more work per warp and
 // no early faces (they were 5 % slower there: other CTAs of the SM fill the wait).
 //
-// Measured on B200 (us per stage; stage kernels / this one), SLAU2, MUSCL:
-//     64 x 33    4.55 / 1.37 (4 rows)
-//    128 x 96    4.32 / 1.37
-//    257 x 131   4.59 / 1.61
-//    333 x 250   5.30 / 2.47
-//    460 x 340    --  / 3.94 (8 rows)
-//    512 x 384   8.02 / 4.63   (42 G cell-stages/s)
-// (8-row tiles where 4 rows fit: 128 x 96 2.4, 257 x 131 2.5, 333 x 250 2.9.)
-// Bound by latency: of about 2600 cycles of a 4-row stage on an idle chip some 1400 pass
+// Measured on B200 (us per stage; stage kernels at their best height / this one), SLAU2,
+// MUSCL:
+//     64 x 33    4.35 / 1.25 (4 rows)
+//    128 x 96    4.12 / 1.25
+//    257 x 131   4.38 / 1.57
+//    300 x 220   4.81 / 2.01
+//    333 x 250   5.09 / 2.46
+//    460 x 340   5.56 / 3.86 (8 rows)
+//    512 x 384   6.98 / 4.48   (44 G cell-stages/s)
+// (8-row tiles where 4 rows fit: 64 x 33 and 128 x 96 2.1, 257 x 131 2.4, 300 x 220 2.5,
+// 333 x 250 2.8.)
+// Bound by latency: of some 2400 cycles of a 4-row stage on an idle chip more than half pass
 // between publishing an edge and having the neighbours' (two L2 trips, with the early
-// faces inside), 600 in one face evaluation and 600 in the combination.  At 512 x 384 the
-// fullest SM holds 6 tiles and issues about 60 % of the time.
+// faces inside), the rest in equal parts in one face evaluation and in the combination.  At
+// 512 x 384 the fullest SM holds 6 tiles and issues about 60 % of the time.
 #include <map>
 #include <mutex>
 #include <type_traits>
@@ -72,9 +75,9 @@ constexpr int RW = 4;  // warps that own cells
 constexpr int aux_warps(int TY) { return TY == 4 ? 2 : 1; }
 // Each height is built twice: for one CTA per SM fewer than would fit, with registers to
 // interleave more of a face's arithmetic, and for all that fit.  A launch takes the first
-// while its tiles fit (us per stage, all that fit / fewer: 128 x 96 1.45 / 1.37, 257 x 131
-// 1.77 / 1.61, 300 x 220 2.14 / 2.04; 8 rows: 460 x 340 4.12 / 3.94, 400 x 380 AUSM+-up
-// 4.37 / 4.09; three CTAs of 4 rows instead of four gain another 1-2 % on the smallest).
+// while its tiles fit (us per stage, all that fit / fewer: 128 x 96 1.33 / 1.25, 257 x 131
+// 1.61 / 1.57, 300 x 220 2.11 / 2.01; 8 rows: 460 x 340 3.99 / 3.86, 400 x 380 AUSM+-up
+// 4.21 / 4.08; three CTAs of 4 rows instead of four gain another 1-2 % on the smallest).
 constexpr int few_ctas(int TY) { return TY == 4 ? 4 : 5; }
 constexpr int more_ctas(int TY) { return TY == 4 ? 5 : 6; }
 constexpr int kMaxTiles4 = more_ctas(4) * 148, kMaxTiles8 = more_ctas(8) * 148;  // tiles of a launch
@@ -410,7 +413,7 @@ __device__ __forceinline__ void resident_tile(Smem<TY>& sm, const Job& b, const 
   }
 }
 
-// OCC: CTAs per SM the registers are sized for (few_ctas and more_ctas below).
+// OCC: CTAs per SM the registers are sized for (few_ctas and more_ctas above).
 template <int SF, int TY, int OCC>
 __global__ void __launch_bounds__(threads_of(TY), OCC)
     k_resident(const float4* Qs, float4* Qo, const float4* __restrict__ Mi, const float4* __restrict__ Mj, float* dt,

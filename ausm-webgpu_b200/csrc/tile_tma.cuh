@@ -125,8 +125,8 @@ __device__ __forceinline__ bool tile_tma_compute(unsigned char* smem, const floa
   const float4 qa = stage_entry(ty + 2, tx + 2);
   const float4 qb = stage_entry(ty + NWY + 2, tx + 2);
   // the halo, its remainder beyond NT entries not on warp 0 either (with the top face row on
-  // the last warp, us per step: 4096 x 3072 606 -> 602, 1155 x 867 55.2 -> 54.1, 700 x 500
-  // 27.1 -> 26.2)
+  // the last warp, us per step: 1155 x 867 55.2 -> 54.1, 700 x 500 27.1 -> 26.2; 4096 x 3072,
+  // whose time the power cap sets, the same within 1 %)
 #pragma unroll
   for (int e = 0; e < (HALO + NT - 1) / NT; e++) {
     const int k = ((tid + NT / 2) & (NT - 1)) + e * NT;

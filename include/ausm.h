@@ -59,8 +59,9 @@ extern "C" {
 #define AUSM_GRID_JACOBI 0
 #define AUSM_GRID_MULTICOLOR 1
 
-/* step engines: one fused kernel per RK stage (default), or the reference's five
- * dispatches per stage (boundary, j-flux, i-flux, residual, RK combine) */
+/* step engines: the fused engine (default: one kernel per RK stage, or all steps of a call in
+ * one launch where the grid fits on the chip), or the reference's operators on its own
+ * layout (boundary and both flux passes in one kernel, residual and RK combine in another) */
 #define AUSM_ENGINE_FUSED 0
 #define AUSM_ENGINE_REFERENCE 1
 #define AUSM_ENGINE_F64 2 /* the reference-shaped engine in FP64 (precision study) */
@@ -153,7 +154,9 @@ int ausm_get_state_f64(ausm_solver* h, double* q);
 
 /* step(n): dt = min(maxdt, cfl / max wave speed) of the current state, held for n
  * TVD-RK3 steps, then the max wave speed of the new state (main.js:744-791).  dt_out
- * may be NULL (then the call does not wait for the GPU).  A tile whose bounded wait
+ * may be NULL (then the call does not wait for the GPU).  The fused engine takes grids up
+ * to 227 K cells by resident launches of up to 360 steps, larger ones by three stage
+ * kernels a step.  A tile whose bounded wait
  * gave up (AUSM_ERR_TIMEOUT) is reported by this call when it waits (dt_out given),
  * else by the next call on the handle that waits for the GPU (get_state, forces,
  * residual_l2, field, max_wave_speed, synchronize, time_steps or a step with dt_out). */
@@ -193,10 +196,11 @@ int ausm_synchronize(ausm_solver* h);
  * on the handle's stream; ms_out gets the elapsed device time of all of them. */
 int ausm_time_steps(ausm_solver* h, int n, int reps, float* ms_out);
 /* Test hook (no counterpart in the reference): the number of polls, 0 to 65536 (the
- * default), of the first bounded wait of every TMA box of the stage kernels on the
- * current device, in this process.  0 makes every such wait give up at once, so a test
- * can drive the timeout path without a fault: the tiles report AUSM_ERR_TIMEOUT, write
- * nothing, and still let their copies land (second wait, full bound) before they exit.
+ * default), of the first bounded wait of every TMA box of the stage kernels, and 64 times
+ * as many of every wait for a neighbour's edge in the resident kernel, on the current
+ * device, in this process.  0 makes every such wait give up at once, so a test can drive
+ * the timeout path without a fault: the tiles report AUSM_ERR_TIMEOUT, write nothing, and
+ * still let their copies land (second wait, full bound) before they exit.
  * The call waits for the device to be idle, so work queued before it keeps the bound it
  * was queued under.  Restore 65536 afterwards. */
 int ausm_debug_set_wait_polls(unsigned polls);
@@ -208,22 +212,30 @@ int ausm_debug_set_exchange_tag(unsigned tag);
 /* Tile-height autotuner of the fused engine (no counterpart in the reference): times
  * the TMA stage kernel for tiles of 32 x 8, 32 x 16 and 32 x 32 cells on this solve's
  * grid and state and keeps the fastest for its steps (cached per M, N and scheme for the
- * process; force = 1 re-measures).  The first ausm_step of an untuned solve runs it
- * implicitly, so call it before capturing steps in a CUDA graph.  AUSM_TILE_ROWS=8|16|32
- * fixes the height, AUSM_AUTOTUNE=0 keeps 16.  *rows gets the height in use. */
+ * process; force = 1 re-measures).  The first ausm_step of an untuned solve above 227 K
+ * cells runs it implicitly; smaller grids, whose steps are resident, use its result in a
+ * stream capture alone (whose steps stay on the stage kernels, at 16 rows if untuned).  It
+ * times and waits, so call it before capturing steps in a CUDA graph: inside a capture it
+ * fails with AUSM_ERR_CUDA.  AUSM_TILE_ROWS=8|16|32 fixes the height and keeps every grid on
+ * the stage kernels, AUSM_AUTOTUNE=0 keeps 16.  *rows gets the height in use. */
 int ausm_autotune(ausm_solver* h, int force, int* rows);
 
 /* ---- batches: many solves advanced together (no counterpart in the reference) ----
  * The reference steps one grid per page.  A batch steps any number of independent
- * fused-engine solvers of any grid sizes and schemes with one kernel launch per RK
- * stage and scheme: the work list is every member's 32 x TY cell tiles end to end (TY
- * chosen by the batch's tile-height tuning), one CTA per tile.  Each
+ * fused-engine solvers of any grid sizes and schemes: in one resident launch of up to 360
+ * steps while the members' tiles all fit on the chip together (227 K cells in all, less
+ * with many ragged grids), else with one kernel launch per RK stage and scheme, whose work
+ * list is every member's 32 x TY cell tiles end to end (TY chosen by the batch's
+ * tile-height tuning), one CTA per tile.  Each
  * member keeps its own dt (from its own max wave speed, held over the n steps as
  * ausm_step does), so a member's results are the same alone or in any batch.  While a
  * solver is a member, its calls run on the batch's stream (ausm_stream returns it) and
  * its engine cannot change; destroying a member removes it first.  A member may belong
- * to one batch.  With graphs on (the default) the n-step sequence is captured once per
- * (membership, n) as a CUDA graph and replayed. */
+ * to one batch.  With graphs on (the default) the n-step sequence of the stage kernels is
+ * captured once per (membership, n) as a CUDA graph and replayed.  With graphs off a host
+ * may capture ausm_batch_step (dt_wave NULL) into a graph of its own: it then stays on the
+ * stage kernels; a direct step must come before it, and again after a change of members or
+ * parameters (AUSM_ERR_STATE, or AUSM_ERR_CUDA where the tile height is still to be tuned). */
 typedef struct ausm_batch ausm_batch;
 /* New empty batch on the current device. */
 int ausm_batch_create(ausm_batch** out);
@@ -240,7 +252,8 @@ int ausm_batch_set_graphs(ausm_batch* b, int enable);
 /* n RK3 steps of every member.  dt_wave (2 floats per member, may be NULL): the dt used
  * and the max wave speed after the steps; with it the call waits for the GPU and
  * returns AUSM_ERR_DIVERGED (after filling dt_wave) when a member's wave speed is not
- * finite.  Without it the call only enqueues the work. */
+ * finite.  Without it the call only enqueues the work.  AUSM_ERR_TIMEOUT is the batch's and
+ * does not say which members' waits gave up: reset every member's state after it. */
 int ausm_batch_step(ausm_batch* b, int n, float* dt_wave);
 /* Density-residual L2 norm of every member's current state (as ausm_residual_l2), one
  * double per member; waits for the GPU. */
@@ -309,7 +322,8 @@ typedef struct AusmServerStats {
 
 typedef struct ausm_server ausm_server;
 /* New server on the current device.  hbm_budget_bytes: device memory its solves may
- * hold at once; max_active: slots (concurrent solves); chunk_steps: RK3 steps per round.
+ * hold at once (the batch's tables and the exchange buffers that all resident launches of
+ * the process share, 10 MiB each and usually one, are not in it); max_active: slots (concurrent solves); chunk_steps: RK3 steps per round.
  * No CUDA call happens until the first round. */
 int ausm_server_create(double hbm_budget_bytes, int max_active, int chunk_steps, int flags, ausm_server** out);
 int ausm_server_destroy(ausm_server* s);
